@@ -5,7 +5,8 @@
 // the Compute kernel of cuda_Cell_Detailed.cu); the line citations are on each
 // function.  Arithmetic is arranged for sm_103a rather than copied: constant
 // divisors become reciprocal multiplies, pow(x, 23) is a product chain,
-// pow(x, 1.787) is exp(1.787 log x), and every quantity that depends only on
+// pow(x, 1.787) is a table-driven power in FP64 and ex2(1.787 lg2 x) in FP32,
+// and every quantity that depends only on
 // the membrane voltage is computed once per cell and step (StepCoef), not per
 // CRU or per channel.
 #pragma once
@@ -14,6 +15,7 @@
 #include <stdint.h>
 
 #include "../../include/rh_philox.h"
+#include "serca_table.cuh"
 
 namespace rh {
 
@@ -185,13 +187,35 @@ __device__ __forceinline__ V vclamp0(V a) {
 }
 
 // SERCA's (x / K)^1.787 for x >= 0 (subroutine_cuda.c:128-146), K = KI_UP
-// for the cytosol (SIDE 0) and KNSR_UP for the network SR (SIDE 1).  FP64 as
-// exp(1.787 log(x / K)); FP32 as ex2(1.787 lg2(x) - 1.787 lg2(K)), the
-// division folded into the constant (lg2(0.123) = -3.0232697793228470,
-// lg2(1700) = 10.731319031025064).
+// for the cytosol (SIDE 0) and KNSR_UP for the network SR (SIDE 1).
+//
+// FP64: bound by the FP64 pipe, where exp(1.787 log(x / K)) costs about 47
+// instructions and a CRU needs sixteen of these powers.  The exponent is
+// fixed, so the power factors over x = 2^e m: with r_i near 1/m from the top
+// seven mantissa bits and t = m r_i - 1 (|t| <= 2^-8, one fma),
+//   (x / K)^a = (2^e / K)^a  r_i^-a  (1 + t)^a,
+// two tabulated factors and the binomial series of (1 + t)^a through t^5
+// (its t^6 term is below 2^-56).  Eight FP64 instructions; the bit fields and
+// the table loads run on other pipes.  Largest error over x in [1e-4, 2e3]:
+// 2.9e-16 relative (the exp(log) form: 3.4e-15).  An x outside [2^-32, 2^32),
+// zero, negative or NaN takes the exp(log) form.
+//
+// FP32: ex2(1.787 lg2(x) - 1.787 lg2(K)), the division folded into the
+// constant (lg2(0.123) = -3.0232697793228470, lg2(1700) =
+// 10.731319031025064).
 template <int SIDE>
 __device__ __forceinline__ double serca_pow(double x) {
-  return Math<double>::powpos(x * (1.0 / (SIDE ? KNSR_UP : KI_UP)), HH_UP);
+  constexpr double A = HH_UP;
+  constexpr double C2 = A * (A - 1) / 2, C3 = C2 * (A - 2) / 3, C4 = C3 * (A - 3) / 4,
+                   C5 = C4 * (A - 4) / 5;
+  const int hi = __double2hiint(x);
+  const uint32_t e = (uint32_t)(hi >> 20) - (1023u - 32u);  // sign set: huge
+  if (e >= 64u) return Math<double>::powpos(x * (1.0 / (SIDE ? KNSR_UP : KI_UP)), HH_UP);
+  const double2 rt = __ldg(&kSercaMant[(hi >> 13) & 127]);
+  const double scale = __ldg(&kSercaExp[SIDE][e]) * rt.y;
+  const double m = __hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(x));
+  const double t = fma(m, rt.x, -1.0);
+  return fma(scale * t, fma(fma(fma(fma(C5, t, C4), t, C3), t, C2), t, A), scale);
 }
 template <int SIDE>
 __device__ __forceinline__ float serca_pow(float x) {

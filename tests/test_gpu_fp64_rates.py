@@ -1,0 +1,46 @@
+"""The FP64 lattice's SERCA and leak rates against numpy over the whole input
+range: table intervals and their edges, powers of two, and the values that
+leave the table (zero, below 2^-32, above 2^32)."""
+import numpy as np
+import pytest
+
+from ryr_hyperactivity_gb300.abi import cell_params
+from ryr_hyperactivity_gb300.sim import Simulator
+
+pytestmark = pytest.mark.gpu
+
+VUP, KI, KNSR, HH = 0.3, 0.123, 1700.0, 1.787  # subroutine_cuda.c:128-146
+GLEAK, KJSR = 0.00001035, 500.0
+
+
+def _inputs(kind, n, rng):
+    if kind == "physiological":
+        return np.exp(rng.uniform(np.log(1e-3), np.log(1e3), n)), rng.uniform(1.0, 2500.0, n)
+    if kind == "interval_edges":  # m at k/128 and one step below, exponents over the table
+        m = 1.0 + rng.integers(0, 128, n) / 128.0
+        x = np.ldexp(m, rng.integers(-12, 12, n))
+        return np.where(np.arange(n) % 2, np.nextafter(x, 0), x), np.ldexp(m, rng.integers(0, 11, n))
+    x = np.ldexp(1.0, rng.integers(-60, 60, n))  # across both ends of the table
+    return np.where(np.arange(n) % 5 == 0, 0.0, x), np.ldexp(1.0 + rng.random(n), rng.integers(-40, 40, n))
+
+
+@pytest.mark.parametrize("kind", ["physiological", "interval_edges", "outside_the_table"])
+def test_fp64_serca_and_leak_match_numpy(kind):
+    p = cell_params(nx=11, ny=7, nz=5, iso2=1, lqt=0)
+    with Simulator(p, precision="fp64") as sim:
+        st = sim.get_state(0)
+        rng = np.random.default_rng(3)
+        ci, cn = _inputs(kind, 8 * st.n, rng)
+        st["ci"][...] = ci
+        st["cnsr"][...] = cn
+        sim.set_state(0, st)
+        sim.lattice_step()
+        got = sim.get_state(0)
+    scale = 1.75 * 1.75 * VUP
+    pa, pb = (ci / KI) ** HH, (cn / KNSR) ** HH
+    up = scale * (pa - pb) / (1 + pa + pb)
+    # a few units in the last place of each power, of their difference's terms
+    # (not of the difference, which cancels) and of the quotient
+    assert np.all(np.abs(got["xiup"] - up) <= 1e-14 * scale * (pa + pb) / (1 + pa + pb))
+    lk = GLEAK * (cn - ci) * cn * cn / (cn * cn + KJSR * KJSR)
+    assert np.all(np.abs(got["xileak"] - lk) <= 1e-14 * np.abs(lk))
