@@ -93,6 +93,45 @@ constexpr double MGI = 500;
 constexpr double VUP = 0.3, KI_UP = 0.123, KNSR_UP = 1700.0, HH_UP = 1.787;
 constexpr double GLEAK = 0.00001035, KJSR_LEAK = 500.0;
 
+// ---- FP64 work kept off the FP64 pipe ----
+//
+// A warp's FP64 instruction occupies this GPU's FP64 pipe 32 times as long as
+// an integer one its own, and the FP64 lattice kernel issues in a tenth of
+// its cycles: tests of a double's sign, range or size are done on its high
+// word with integer instructions.
+
+// Exponent field 0 or 0x7ff: zero, subnormal, infinite or NaN.
+__device__ __forceinline__ bool extreme(double x) {
+  return ((__double2hiint(x) + 0x00100000) & 0x7fe00000) == 0;
+}
+
+// Reciprocal of d from the hardware's rough reciprocal y0 (measured: off by
+// at most 2^-19.9) by one third-order step: with e = 1 - d y0, 1/d =
+// y0 (1 + e + e^2 + ...) and y0 (1 + e + e^2) is off by e^3 (Householder's
+// iteration for 1/d; measured 1.1e-16 at most).  Not for d or 1/d zero,
+// subnormal or infinite: the caller tests `extreme` on the seed.
+__device__ __forceinline__ double rcp_seed(double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  return y;
+}
+__device__ __forceinline__ double rcp_refine(double d, double y) {
+  const double e = fma(-d, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+// a / b in six FP64 instructions: the reciprocal, the quotient and one
+// residual correction of it (equal to the rounded quotient in 39 million
+// random pairs).  A seed or quotient outside the normal range
+// takes the ordinary division.
+__device__ __forceinline__ double div_refined(double a, double b) {
+  const double y0 = rcp_seed(b);
+  const double y = rcp_refine(b, y0);
+  const double q = a * y;
+  if (extreme(y0) || extreme(q)) return a / b;
+  return fma(fma(-b, q, a), y, q);
+}
+
 // ---- math of each precision ----
 template <class R>
 struct Math;
@@ -108,7 +147,7 @@ struct Math<double> {
   static __device__ __forceinline__ double powpos(double x, double y) {
     return ::exp(y * ::log(x));
   }
-  static __device__ __forceinline__ double div(double a, double b) { return a / b; }
+  static __device__ __forceinline__ double div(double a, double b) { return div_refined(a, b); }
   static __device__ __forceinline__ int to_int(double x) { return __double2int_rz(x); }
   static __device__ __forceinline__ double uniform(rh_stream* s) { return rh_uniform_double(s); }
   static constexpr double TINY_UNIFORM = 0x1.0p-53;
@@ -172,13 +211,16 @@ __device__ __forceinline__ double2 vfma(double2 a, double2 b, double2 c) {
 __device__ __forceinline__ double2 vsub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 // x < 0 ? 0 : x, NaN staying NaN.  In FP32 one max.NaN instruction (its
 // max(-0, +0) is +0 where the comparison keeps -0, which no later FP32 result
-// tells apart); in FP64 the comparison itself, as the oracle has it.
+// tells apart); in FP64 an integer test of the high word (-0 to -inf: sign
+// set, at most the infinity's word), which likewise makes -0 a +0.
 __device__ __forceinline__ float clamp0(float x) {
   float r;
   asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(x));
   return r;
 }
-__device__ __forceinline__ double clamp0(double x) { return x < 0.0 ? 0.0 : x; }
+__device__ __forceinline__ double clamp0(double x) {
+  return ((uint32_t)__double2hiint(x) ^ 0x80000000u) <= 0x7ff00000u ? 0.0 : x;
+}
 template <class V>
 __device__ __forceinline__ V vclamp0(V a) {
   a.x = clamp0(a.x);
@@ -223,6 +265,30 @@ __device__ __forceinline__ float serca_pow(float x) {
   return ex2_approx(fmaf((float)HH_UP, __log2f(x), (float)(-HH_UP * lg2k)));
 }
 
+// SERCA uptake and leak of one sub-voxel (subroutine_cuda.c:128-146): up =
+// sviup VUP (pa - pb) / (1 + pa + pb) and lk = GLEAK (n - c) n^2 / (n^2 +
+// KJSR_LEAK^2), with pa and pb the SERCA powers of c and n.
+// FP64: both quotients share one reciprocal, 1/(d1 d2), and each takes its
+// own residual correction.
+__device__ __forceinline__ void serca_leak(double c, double n, double pa, double pb, double sviup,
+                                           double& up, double& lk) {
+  const double nu = VUP * (pa - pb), d1 = 1.0 + pa + pb;
+  const double n2 = n * n;
+  const double nl = GLEAK * (n - c) * n2, d2 = n2 + KJSR_LEAK * KJSR_LEAK;
+  const double d = d1 * d2;
+  const double y0 = rcp_seed(d);
+  if (extreme(y0) || extreme(d1) || extreme(d2)) {
+    up = sviup * (nu / d1);
+    lk = nl / d2;
+    return;
+  }
+  const double y = rcp_refine(d, y0);
+  const double y1 = d2 * y, y2 = d1 * y;
+  const double q1 = nu * y1, q2 = nl * y2;
+  up = sviup * fma(fma(-d1, q1, nu), y1, q1);
+  lk = fma(fma(-d2, q2, nl), y2, q2);
+}
+
 template <class R>
 __device__ __forceinline__ R pow23(R x) {  // x^23 = x^16 x^4 x^2 x
   R x2 = x * x, x4 = x2 * x2, x8 = x4 * x4, x16 = x8 * x8;
@@ -231,13 +297,29 @@ __device__ __forceinline__ R pow23(R x) {  // x^23 = x^16 x^4 x^2 x
 
 // ---- buffers (buffers.c:55-155) ----
 
+// The reference's saturation guard on * dt > 1 of an on-rate `on` (buffers.c).
+// FP64: `hr` is the high word of 1/dt (within a few units in its last place);
+// an on-rate whose high word is more than one step away from it lies on a
+// known side, so the product and the FP64 comparison run for one value in
+// 2^18.  `hr` is not used in FP32.
+__device__ __forceinline__ bool saturates(float on, float dt, int) { return on * dt > 1.0f; }
+__device__ __forceinline__ bool saturates(double on, double dt, int hr) {
+  const int h = __double2hiint(on);
+  if (h < hr - 1) return false;  // also every negative on
+  if ((uint32_t)(h - (hr + 2)) <= 0x7ff00000u - (uint32_t)(hr + 2)) return true;  // to +inf
+  return on * dt > 1.0;  // close to 1/dt, or NaN
+}
+__device__ __forceinline__ int guard_word(float) { return 0; }
+__device__ __forceinline__ int guard_word(double rdt) { return __double2hiint(rdt); }
+
 // Mass-action rate with the reference's saturation guard kon*c*dt > 1, which
 // replaces the on-rate kon*c by 0.95/dt: the guard selects the factor, one
 // expression computes the rate.
 template <class R>
-__device__ __forceinline__ R buffer_rate(R kon, R koff, R total, R bound, R c, R dt, R rdt95) {
+__device__ __forceinline__ R buffer_rate(R kon, R koff, R total, R bound, R c, R dt, int hr,
+                                         R rdt95) {
   R on = kon * c;
-  on = (on * dt > R(1)) ? rdt95 : on;
+  on = saturates(on, dt, hr) ? rdt95 : on;
   return on * (total - bound) - koff * bound;
 }
 
@@ -253,8 +335,8 @@ __device__ __forceinline__ void csqn_mono(R cjsr, R& roo2, R& mono);
 
 template <>
 __device__ __forceinline__ void csqn_mono<double>(double cjsr, double& roo2, double& mono) {
-  roo2 = RATEDIMER / (1.0 + pow23(KDIMER / cjsr));
-  mono = (-1.0 + ::sqrt(1.0 + 8.0 * CSQBERS * roo2)) / (4.0 * roo2 * CSQBERS);
+  roo2 = div_refined(RATEDIMER, 1.0 + pow23(div_refined(KDIMER, cjsr)));
+  mono = div_refined(-1.0 + ::sqrt(1.0 + 8.0 * CSQBERS * roo2), 4.0 * roo2 * CSQBERS);
 }
 
 template <>

@@ -688,7 +688,8 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
     if (prevsp < 5 && nou + nob >= 5) nspark = 1;
     const R po = Math<R>::div(R(nou + nob), R(NRYR));
     R xire = R(0.0147 * SVJMAX) * po * (cjsr - cp) * R(1.0 / VP);
-    xire = clamp0(xire);
+    if (sizeof(R) == 8) xire = xire < R(0) ? R(0) : xire;  // keeps the -0 the records print
+    else xire = clamp0(xire);
 
     // ---- NCX (:1296, subroutine_cuda.c:47-120); zero in a permeabilised
     //      cell, whose Ancx keeps its value (:1302) ----
@@ -740,6 +741,7 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
     R csn = cs0;
     {
       const R dth = k.dth, rdth95 = k.rdth95;
+      const int hrh = guard_word(R(5) * k.rdt);  // 1/dth
       // z faces: zero flux (the ghost repeats cs), or the permeabilised
       // cell's bath value, which its ghosts keep (:1603-1689 under -Dperm)
       const R cs_face = o_perm ? R(PERM_CI_BASAL) : cs0;
@@ -754,14 +756,14 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
           (ci0 - cp) * R(1.0 / TAUPI / 2.) + (ci1 - cp) * R(1.0 / TAUPI / 2.) + xire - icat1;
 #pragma unroll 1
       for (int it = 0; it < 5; ++it) {
-        const R r_sar = buffer_rate<R>(R(KSARON), R(KSAROFF), R(BSAR), casar, csn, dth, rdth95);
+        const R r_sar = buffer_rate<R>(R(KSARON), R(KSAROFF), R(BSAR), casar, csn, dth, hrh, rdth95);
         const R r_sarh =
-            buffer_rate<R>(R(KSARHON), R(KSARHOFF), R(BSARH), casarh, csn, dth, rdth95);
+            buffer_rate<R>(R(KSARHON), R(KSARHOFF), R(BSARH), casarh, csn, dth, hrh, rdth95);
         R dotcs = R(VP / VS / TAUPS) * (cp - csn) + cs_const - (r_sar + r_sarh);
         if (o_perm) dotcs += (R(PERM_CI_BASAL) - csn) * R(0.2);  // :1409-1411
-        const R cpbuff = buffer_rate<R>(R(KSARON), R(KSAROFF), R(BSAR), casarj, cp, dth, rdth95);
+        const R cpbuff = buffer_rate<R>(R(KSARON), R(KSAROFF), R(BSAR), casarj, cp, dth, hrh, rdth95);
         const R cpbuffh =
-            buffer_rate<R>(R(KSARHON), R(KSARHOFF), R(BSARH), casarhj, cp, dth, rdth95);
+            buffer_rate<R>(R(KSARHON), R(KSARHOFF), R(BSARH), casarhj, cp, dth, hrh, rdth95);
         const R cpdot = (csn - cp) * R(1.0 / TAUPS) + cp_const - cpbuff - cpbuffh;
         casarj = clamp0(casarj + cpbuff * dth);
         casarhj = clamp0(casarhj + cpbuffh * dth);
@@ -819,6 +821,8 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
     const V kt_n = splat2(R(1.0 / (TAUNT * XI))), kl_n = splat2(R(1.0 / (TAUNL * XI)));
     const V kt_i = splat2(R(1.0 / (TAUIT * XI))), kl_i = splat2(R(1.0 / (TAUIL * XI)));
     const V dt2 = splat2(dt);
+    const int hr = guard_word(k.rdt);
+    const int hrs = guard_word(k.rdt * R(1.0 / KSRON));  // c above which the SR buffer saturates
     const V* catf2 = reinterpret_cast<const V*>(L.catf);
     const V* cats2 = reinterpret_cast<const V*>(L.cats);
     const V* cacal2 = reinterpret_cast<const V*>(L.cacal);
@@ -956,12 +960,17 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
       {
         const R pax = serca_pow<0>(c.x), pay = serca_pow<0>(c.y);
         const R pbx = serca_pow<1>(n.x), pby = serca_pow<1>(n.y);
-        up = v2(k.sviup * Math<R>::div(R(VUP) * (pax - pbx), R(1) + pax + pbx),
-                k.sviup * Math<R>::div(R(VUP) * (pay - pby), R(1) + pay + pby));
-        const V n2 = vmul(n, n);
-        const V num = vmul(vmul(splat2(R(GLEAK)), vsub(n, c)), n2);
-        const V den = vadd(n2, splat2(R(KJSR_LEAK * KJSR_LEAK)));
-        lk = v2(Math<R>::div(num.x, den.x), Math<R>::div(num.y, den.y));
+        if constexpr (sizeof(R) == 8) {
+          serca_leak(c.x, n.x, pax, pbx, k.sviup, up.x, lk.x);
+          serca_leak(c.y, n.y, pay, pby, k.sviup, up.y, lk.y);
+        } else {
+          up = v2(k.sviup * Math<R>::div(R(VUP) * (pax - pbx), R(1) + pax + pbx),
+                  k.sviup * Math<R>::div(R(VUP) * (pay - pby), R(1) + pay + pby));
+          const V n2 = vmul(n, n);
+          const V num = vmul(vmul(splat2(R(GLEAK)), vsub(n, c)), n2);
+          const V den = vadd(n2, splat2(R(KJSR_LEAK * KJSR_LEAK)));
+          lk = v2(Math<R>::div(num.x, den.x), Math<R>::div(num.y, den.y));
+        }
       }
       // cytosolic buffers (buffers.c:55-115): on*(B-b) - koff*b, where the
       // saturation guard kon*c*dt > 1 replaces on by 0.95/dt.  Myosin's
@@ -976,11 +985,13 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
                      vmul(splat2(R(-KCALOFF)), cacal));
       V r_sr = vfma(vmul(splat2(R(KSRON)), c), vsub(splat2(R(BSR)), casr), vmul(splat2(R(-KSROFF)), casr));
       V on_mc = vmul(splat2(R(KONMYOCA)), c);
-      on_mc.x = (on_mc.x * dt > R(1)) ? k.rdt95 : on_mc.x;
-      on_mc.y = (on_mc.y * dt > R(1)) ? k.rdt95 : on_mc.y;
+      on_mc.x = saturates(on_mc.x, dt, hr) ? k.rdt95 : on_mc.x;
+      on_mc.y = saturates(on_mc.y, dt, hr) ? k.rdt95 : on_mc.y;
       const V r_mc = vfma(on_mc, freemyo, vmul(splat2(R(-KOFFMYOCA)), camyo));
       static_assert(KTFON <= KSRON && KTSON <= KSRON && KCALON <= KSRON, "SR has the largest on-rate");
-      if (fmax(c.x, c.y) * R(KSRON) * dt > R(1)) {  // another buffer saturates
+      // another buffer saturates (FP64: may saturate, by the high words)
+      if (sizeof(R) == 8 ? max(guard_word(c.x), guard_word(c.y)) >= hrs - 1
+                         : fmax(c.x, c.y) * R(KSRON) * dt > R(1)) {
         const R cc[2] = {c.x, c.y};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -989,10 +1000,10 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
           R& ts = h ? r_ts.y : r_ts.x;
           R& cal = h ? r_cal.y : r_cal.x;
           R& sr = h ? r_sr.y : r_sr.x;
-          tf = buffer_rate<R>(R(KTFON), R(KTFOFF), R(BTF), h ? catf.y : catf.x, cv, dt, k.rdt95);
-          ts = buffer_rate<R>(R(KTSON), R(KTSOFF), R(BTS), h ? cats.y : cats.x, cv, dt, k.rdt95);
-          cal = buffer_rate<R>(R(KCALON), R(KCALOFF), R(BCAL), h ? cacal.y : cacal.x, cv, dt, k.rdt95);
-          sr = buffer_rate<R>(R(KSRON), R(KSROFF), R(BSR), h ? casr.y : casr.x, cv, dt, k.rdt95);
+          tf = buffer_rate<R>(R(KTFON), R(KTFOFF), R(BTF), h ? catf.y : catf.x, cv, dt, hr, k.rdt95);
+          ts = buffer_rate<R>(R(KTSON), R(KTSOFF), R(BTS), h ? cats.y : cats.x, cv, dt, hr, k.rdt95);
+          cal = buffer_rate<R>(R(KCALON), R(KCALOFF), R(BCAL), h ? cacal.y : cacal.x, cv, dt, hr, k.rdt95);
+          sr = buffer_rate<R>(R(KSRON), R(KSROFF), R(BSR), h ? casr.y : casr.x, cv, dt, hr, k.rdt95);
         }
       }
       V dotcn = vfma(vsub(up, lk), splat2(R(VI / VNSR)), coupn);
