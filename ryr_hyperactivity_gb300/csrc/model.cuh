@@ -450,16 +450,18 @@ __device__ __forceinline__ int ryr_transition(rh_stream* rng, int n, R p, R lam,
   return m;
 }
 
-// Four-state RyR cluster step (subroutine_cuda.c:251-669).  roo2/mono come
-// from csqn_mono (the same expression the reference evaluates at :328-329).
-// The eight transitions run in source order (so do their draws), unrolled:
-// each transition's count and rates are then fixed at compile time, which
-// measured 1% faster than the rolled loop despite the larger code; each count
-// is packed into a byte (counts are <= 195 before clamping).
-template <class R>
-__device__ __forceinline__ void ryr_gating(rh_stream* rng, const StepCoef<R>& k, R cp, R cjsr,
-                                           R mono, int& ncu, int& nou, int& ncb, int& nob,
-                                           uint32_t* status) {
+// The eight transition counts of a RyR cluster step (subroutine_cuda.c:
+// 251-613), four to a word.  roo2/mono come from csqn_mono (the same
+// expression the reference evaluates at :328-329).  The transitions run in
+// source order (so do their draws); each count is packed into a byte (counts
+// are <= 195 before clamping).  UNROLL 8 fixes each transition's count and
+// rates at compile time, which measured 1% faster than the rolled loop in the
+// FP32 kernel despite the larger code.
+template <class R, int UNROLL>
+__device__ __forceinline__ void ryr_draws(rh_stream* rng, const StepCoef<R>& k, R cp, R cjsr,
+                                          R mono, int nou0, int ncu0, int nob0, int ncb0,
+                                          uint32_t& packed0, uint32_t& packed1,
+                                          uint32_t* status) {
   const R dt = k.dt;
   R q = Math<R>::div(R(5000), cjsr);
   R a = Math<R>::div(k.ku, cp);
@@ -474,11 +476,11 @@ __device__ __forceinline__ void ryr_gating(rh_stream* rng, const StepCoef<R>& k,
   if (pkbminus * dt > R(1)) pkbminus = k.rdt;
   const R aub = mono * R(1.0 / TAUB);
   const R abu = R(1.0 / TAUU);
-  const int nou0 = nou, ncu0 = ncu, nob0 = nob, ncb0 = ncb;
   const R pbu = (pkb < R(1e-16)) ? abu * dt * R(36) : abu * dt * Math<R>::div(pku, pkb);
   const R pau = (pkb < R(1e-16)) ? R(0) : aub * dt;
-  uint32_t packed0 = 0u, packed1 = 0u;
-#pragma unroll
+  packed0 = 0u;
+  packed1 = 0u;
+#pragma unroll UNROLL
   for (int t = 0; t < 8; ++t) {
     int n;
     R p;
@@ -497,6 +499,103 @@ __device__ __forceinline__ void ryr_gating(rh_stream* rng, const StepCoef<R>& k,
     r = min(r, 255);
     if (t < 4) packed0 |= (uint32_t)r << (t * 8);
     else packed1 |= (uint32_t)r << ((t - 4) * 8);
+  }
+}
+
+// ---- the FP64 lattice's channel draws, decided in FP32 ----
+//
+// A draw compares FP64 uniforms with FP64 rates; the outcome is an integer.
+// FP32 estimates of both sides decide it wherever they differ by more than
+// the estimates' error, and only a CRU with a closer comparison (about one
+// warp in a hundred has one) repeats its draws in FP64: the counts are those
+// of the FP64 comparison in every case.  That takes the eight exponentials,
+// the rates' divisions and the uniforms' conversions off the FP64 pipe, which
+// bounds this kernel.
+
+// x truncated to FP32 by its bits (below 2^-23 relative): nothing of it runs
+// on the FP64 pipe.  Tiny x gives 0; a negative, large (>= 2^127) or NaN x
+// clears `ok`.
+__device__ __forceinline__ float narrow(double x, bool& ok) {
+  const int hi = __double2hiint(x);
+  ok = ok && (uint32_t)hi < (1150u << 20);
+  const uint32_t b = __funnelshift_l((uint32_t)__double2loint(x), (uint32_t)hi - 0x38000000u, 3);
+  return hi < (897 << 20) ? 0.0f : __uint_as_float(b);
+}
+
+// The stream's next uniform to FP32: within 2^-32 + 2^-24 u of the FP64 one.
+__device__ __forceinline__ float uniform_estimate(rh_stream* rng) {
+  uint32_t hi, lo;
+  rh_stream_next(rng, &hi, &lo);
+  return __uint2float_rn(hi) * 0x1.0p-32f;
+}
+
+// ryr_draws<double> with every comparison decided in FP32; false (the counts
+// and the stream are then to be discarded) where one is too close, where a
+// transition might take the Gaussian branch, or where an input is out of
+// FP32's range.  Error of n p: 3e-6 relative (truncated inputs, the squares
+// of two quotients); of exp(-n p): that and __expf's 3e-7 + 1.4e-7 n p; of a
+// product of kk uniforms: kk (2^-32 + 1.2e-7 of its value), kk <= 32.
+__device__ __forceinline__ bool ryr_draws_estimated(rh_stream* rng, const StepCoef<double>& k,
+                                                    double cp, double cjsr, double mono, int nou0,
+                                                    int ncu0, int nob0, int ncb0,
+                                                    uint32_t& packed0, uint32_t& packed1) {
+  bool ok = true;
+  const float dt = narrow(k.dt, ok);
+  const float q = __fdividef(5000.0f, narrow(cjsr, ok));
+  const float a = __fdividef(narrow(k.ku, ok), narrow(cp, ok));
+  const float common = __fdividef(1.0f, (1.0f + q * q) * (1.0f + a * a));
+  const float step = fminf(dt, 1.0f);  // the rates of 1 per ms, capped
+  const float pku = fminf(float(4.5 * 1.5) * narrow(k.ku2, ok) * common * dt, 1.0f);
+  const float pkb0 = float(4.5 * 1.5 / 36.) * narrow(k.kb, ok) * common;
+  const float pkb = fminf(pkb0 * dt, 1.0f);
+  const float aub = narrow(mono, ok) * float(1.0 / TAUB) * dt;
+  const float abu = float(1.0 / TAUU) * dt;
+  const bool unbound = pkb0 < 1e-16f;
+  ok = ok && !(pkb0 > 0.99e-16f && pkb0 < 1.01e-16f);
+  const float pbu = unbound ? abu * 36.0f : abu * __fdividef(pku, pkb);
+  const float pau = unbound ? 0.0f : aub;
+  packed0 = 0u;
+  packed1 = 0u;
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+    const int n = t == 0 || t == 2 ? nou0 : t == 1 || t == 5 ? ncu0 : t == 3 || t == 6 ? nob0 : ncb0;
+    const float p = t == 0 || t == 6 ? step : t == 1 ? pku : t == 2 ? pau : t == 3 ? pbu
+                  : t == 4 ? abu : t == 5 ? aub : pkb;
+    const float s = (float)n * p;
+    ok = ok && s >= 0.0f && (n <= 1 || p < 0.1999f);
+    const float lam = __expf(-s);
+    const float tol = fmaf(lam, fmaf(s, 6e-6f, 8e-6f), 2e-8f);
+    float puu = 1.0f, d;
+    int kk = 0;
+    do {
+      ++kk;
+      puu *= uniform_estimate(rng);
+      d = puu - lam;
+      ok = ok && fabsf(d) > tol && kk < 32;
+    } while (d > 0.0f && ok);
+    if (!ok) return false;
+    if (t < 4) packed0 |= (uint32_t)(kk - 1) << (t * 8);
+    else packed1 |= (uint32_t)(kk - 1) << ((t - 4) * 8);
+  }
+  return true;
+}
+
+// Four-state RyR cluster step (subroutine_cuda.c:251-669): the transition
+// counts, then the conflicts among them and the new occupancies.
+template <class R>
+__device__ __forceinline__ void ryr_gating(rh_stream* rng, const StepCoef<R>& k, R cp, R cjsr,
+                                           R mono, int& ncu, int& nou, int& ncb, int& nob,
+                                           uint32_t* status) {
+  const int nou0 = nou, ncu0 = ncu, nob0 = nob, ncb0 = ncb;
+  uint32_t packed0, packed1;
+  if constexpr (sizeof(R) == 8) {
+    const rh_stream at = *rng;
+    if (!ryr_draws_estimated(rng, k, cp, cjsr, mono, nou0, ncu0, nob0, ncb0, packed0, packed1)) {
+      *rng = at;
+      ryr_draws<R, 1>(rng, k, cp, cjsr, mono, nou0, ncu0, nob0, ncb0, packed0, packed1, status);
+    }
+  } else {
+    ryr_draws<R, 8>(rng, k, cp, cjsr, mono, nou0, ncu0, nob0, ncb0, packed0, packed1, status);
   }
   int n_ou_cu = packed0 & 0xff, n_cu_ou = (packed0 >> 8) & 0xff;
   int n_ou_ob = (packed0 >> 16) & 0xff, n_ob_ou = packed0 >> 24;
@@ -545,6 +644,65 @@ __device__ __forceinline__ int lcc_next(int st, R rig, R ac, R bc, R ad, R bd, R
   const R g1 = rig - r0, g2 = g1 - r1, g3 = g2 - r2;
   const int flip = rig < r0 ? 1 : g1 < r1 ? 2 : g2 < r2 ? 4 : g3 < r3 ? 8 : 0;
   return st ^ flip;
+}
+
+// A CRU's LCC slots (cuda_Cell_Detailed.cu:1248-1263): one uniform and at
+// most one flip each, up to the first empty slot (16); the channels left in
+// state 0 are counted in `open` and in the window counter nl.  bfca is the
+// Ca-dependent inactivation rate.
+template <class R>
+__device__ __forceinline__ void lcc_slots(rh_stream* rng, uint64_t& slots, const StepCoef<R>& k,
+                                          R bfca, int& nl, int& open) {
+#pragma unroll 1
+  for (int ll = 0; ll < 8; ++ll) {
+    const int sh8 = ll * 8;
+    int st = (int)((slots >> sh8) & 0xff);
+    if (st >= 16) break;  // the reference stops at the first empty slot
+    R u = Math<R>::uniform(rng);
+    st = lcc_next<R>(st, u * k.rdt, k.alphac, k.betac, k.alphad, k.betad, k.alphaf, k.betaf,
+                     R(0.012 / 2.), bfca);
+    slots = (slots & ~(0xffull << sh8)) | ((uint64_t)st << sh8);
+    if (st == 0) {
+      ++nl;
+      ++open;
+    }
+  }
+}
+
+// The inactivation rate (reesica.h:57-63).
+template <class R>
+__device__ __forceinline__ R lcc_bfca(R cpx) {
+  const R qq = Math<R>::div(R(25), cpx);
+  return Math<R>::div(R(0.175), R(1) + qq * qq);
+}
+
+// lcc_slots<double> decided in FP32, as ryr_draws_estimated: false where a
+// passage is within the estimates' error, 1e-6 of the largest term.
+__device__ __forceinline__ bool lcc_slots_estimated(rh_stream* rng, uint64_t& slots,
+                                                    const StepCoef<double>& k, double cpx,
+                                                    int& nl, int& open) {
+  bool ok = true;
+  const float rdt = narrow(k.rdt, ok);
+  const float ac = narrow(k.alphac, ok), bc = narrow(k.betac, ok), ad = narrow(k.alphad, ok);
+  const float bd = narrow(k.betad, ok), af = narrow(k.alphaf, ok), bf = narrow(k.betaf, ok);
+  const float bfca = lcc_bfca<float>(narrow(cpx, ok));
+  const float tol = 1e-6f * (rdt + ac + bc + ad + bd + af + bf);
+#pragma unroll 1
+  for (int ll = 0; ll < 8; ++ll) {
+    const int sh8 = ll * 8;
+    int st = (int)((slots >> sh8) & 0xff);
+    if (st >= 16) break;
+    const float g0 = uniform_estimate(rng) * rdt - ((st & 1) ? ac : bc);
+    const float g1 = g0 - ((st & 2) ? ad : bd), g2 = g1 - ((st & 4) ? af : bf);
+    const float g3 = g2 - ((st & 8) ? float(0.012 / 2.) : bfca);
+    ok = ok && fminf(fminf(fabsf(g0), fabsf(g1)), fminf(fabsf(g2), fabsf(g3))) > tol;
+    if (!ok) return false;
+    st ^= g0 < 0.0f ? 1 : g1 < 0.0f ? 2 : g2 < 0.0f ? 4 : g3 < 0.0f ? 8 : 0;
+    slots = (slots & ~(0xffull << sh8)) | ((uint64_t)st << sh8);
+    if (st == 0) ++open;
+  }
+  nl += open;
+  return true;
 }
 
 }  // namespace rh

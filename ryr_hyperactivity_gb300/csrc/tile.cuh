@@ -641,11 +641,7 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
 
     // ---- LCC channels (:1248-1263, reesica.h:14-116) ----
     const R cpx = Math<R>::div(cp + cs0 * R(ICAGAMMA), R(1 + ICAGAMMA));
-    R bfca;
-    {
-      R qq = Math<R>::div(R(25), cpx);
-      bfca = Math<R>::div(R(0.175), R(1) + qq * qq);
-    }
+    const R bfca = sizeof(R) == 4 ? lcc_bfca<R>(cpx) : R(0);  // FP64: only for repeated draws
     if (OPT && k.iso_add_lcc) {  // iso: the empty slots 4-7 receive a channel in state 3 (:1213-1218)
       uint32_t hi = lccw.y;
 #pragma unroll
@@ -656,19 +652,16 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
     int nlcp = 0;
     if (!o_perm) {  // a permeabilised cell has no LCC current (:1249-1263 under -Dperm)
       uint64_t slots = ((uint64_t)lccw.y << 32) | lccw.x;
-#pragma unroll 1
-      for (int ll = 0; ll < 8; ++ll) {
-        const int sh8 = ll * 8;
-        int st = (int)((slots >> sh8) & 0xff);
-        if (st >= 16) break;  // the reference stops at the first empty slot
-        R u = Math<R>::uniform(&rng);
-        st = lcc_next<R>(st, u * k.rdt, k.alphac, k.betac, k.alphad, k.betad, k.alphaf, k.betaf,
-                         R(0.012 / 2.), bfca);
-        slots = (slots & ~(0xffull << sh8)) | ((uint64_t)st << sh8);
-        if (st == 0) {
-          ++nl;
-          ++nlcp;
+      if constexpr (sizeof(R) == 8) {
+        const uint64_t slots0 = slots;
+        if (!lcc_slots_estimated(&rng, slots, k, cpx, nl, nlcp)) {
+          rng.draw = 0u;
+          slots = slots0;
+          nlcp = 0;
+          lcc_slots<R>(&rng, slots, k, lcc_bfca<R>(cpx), nl, nlcp);
         }
+      } else {
+        lcc_slots<R>(&rng, slots, k, bfca, nl, nlcp);
       }
       lccw.x = (uint32_t)slots;
       lccw.y = (uint32_t)(slots >> 32);

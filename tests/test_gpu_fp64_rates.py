@@ -44,3 +44,37 @@ def test_fp64_serca_and_leak_match_numpy(kind):
     assert np.all(np.abs(got["xiup"] - up) <= 1e-14 * scale * (pa + pb) / (1 + pa + pb))
     lk = GLEAK * (cn - ci) * cn * cn / (cn * cn + KJSR * KJSR)
     assert np.all(np.abs(got["xileak"] - lk) <= 1e-14 * np.abs(lk))
+
+
+@pytest.mark.parametrize("seed,v,params", [
+    (0, -80.0, dict()), (1, 0.5, dict(ku2=3.0)), (2, 30.0, dict(kb=0.0)), (3, -40.0, dict(ku=0.5, ku2=3.0)),
+])
+def test_fp64_channel_draws_are_those_of_the_fp64_comparisons(seed, v, params):
+    """The FP64 lattice decides most draws from FP32 estimates and repeats the
+    close ones in FP64: over half a million draws at rates from zero to the
+    Gaussian branch, every count equals the oracle's."""
+    from oracle import oracle as O
+    from tests.gpu_helpers import count_mismatch
+
+    p = cell_params(nx=100, ny=30, nz=20, lqt=0, seed=seed, **params)
+    o = O.Oracle(p)
+    st, m = o.get_state(), o.get_membrane()
+    rng = np.random.default_rng(seed)
+    st["cp"][...] = np.exp(rng.uniform(np.log(1e-2), np.log(300.0), st.n))
+    st["cp"][::97] = 0.0
+    st["cjsr"][...] = rng.uniform(20.0, 1500.0, st.n)
+    occ = rng.multinomial(100, [0.02, 0.5, 0.03, 0.45], st.n)
+    for i, f in enumerate(["nou", "ncu", "nob", "ncb"]):
+        st[f][...] = occ[:, i]
+    st["lcc"].reshape(8, -1)[:4] = rng.integers(0, 16, (4, st.n))
+    m.v = v
+    o.set_state(st)
+    o.set_membrane(m)
+    o.lattice_step()
+    with Simulator(p, precision="fp64") as sim:
+        sim.set_state(0, st)
+        sim.set_membrane(0, m)
+        sim.lattice_step()
+        got = sim.get_state(0)
+    bad = count_mismatch(got, o.get_state())
+    assert not bad.any(), np.flatnonzero(bad)[:10]
