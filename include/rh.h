@@ -328,7 +328,10 @@ typedef struct {
   int32_t persistent;   /* 1 = one persistent cooperative launch per window,
                            0 = two launches per step and cell group */
   int32_t tile_crus;    /* CRUs (threads) per CTA: 64, 128 or 256; the
-                           persistent launch takes 64 or 128 */
+                           persistent launch takes 64 or 128.  While no shape
+                           was asked for (block_size 0, no rh_set_launch_shape
+                           or autotuner), small lattices run one-warp CTAs
+                           instead, with the same results */
   int32_t fewer_ctas;   /* persistent launch only: 1 = one resident CTA per SM
                            fewer than the step kernel holds, with more registers
                            per thread (cells without build options only) */

@@ -35,7 +35,8 @@ struct rh_sim {
   rh_run_opts opts{};
   std::vector<rh_cell_params> params;
   std::vector<CellConst> hcells;  // per-cell constants (tile fields of the current set)
-  // one tile table per compiled tile length (kTileSizes); `ts` is in use
+  // one tile table per compiled tile length (kTileSizes, then the narrow
+  // tiles); `ts` is the launch shape's, active_set() the one in use
   struct TileSet {
     int tile = 0;
     int ntiles = 0;
@@ -43,8 +44,10 @@ struct rh_sim {
     std::vector<int4> htiles;
     CellConst* d_cells = nullptr;
     int4* d_tiles = nullptr;
-  } sets[kNumTileSizes];
+  } sets[kNumTileSets];
   int ts = 0;
+  bool shape_given = false;  // a tile length was asked for (run option, launch shape, autotuner)
+  int sm_count = 0;
   // Cell groups: contiguous cell ranges of about equal CRU count, each with
   // its own stream.  A window of steps runs as one graph with a branch per
   // group, so one group's end-of-step tail (its last lattice CTAs and its
@@ -291,13 +294,38 @@ size_t lattice_bytes(size_t rs, int64_t S) {
   return 10 * al(S * rs) + 10 * al(8 * S * rs) + al(S * 4) + al(S * 8) + al(S * 4);
 }
 
+// Whether windows of steps run as one persistent launch: the run option, a
+// tile length the window kernel is compiled for, and a device that can
+// launch it cooperatively.
+bool use_persist(const rh_sim* s) {
+  const int tile = s->sets[s->ts].tile;
+  return s->opts.persistent && s->persist_ok && (tile == 64 || tile == 128);
+}
+
+// The tile table the two-launch path runs: the launch shape's, or the narrow
+// tiles (one warp per CTA) where no shape was asked for and one wave of warps
+// holds the whole lattice.  128-CRU tiles then leave SMs without work: a
+// 100x20x10 cell fills 111 of 152.  FP64, up to the 12 warps an SM holds (a
+// warp's rate is set by its scheduler's FP64 unit, so warps want spreading):
+// per 100 steps, one 20x10x5 cell 6.39 ms against 6.57, one 100x20x10 cell
+// 7.06 against 7.40, ten 3,705-CRU cells 10.16 against 10.75.  FP32, up to one
+// warp per scheduler: one 100x20x10 cell 2.33 against 2.37 ms, but 200 cells of
+// 432 CRUs (18 warps per SM) 3.68 against 2.91: four-warp CTAs share their
+// header, staging and barriers.
+int active_set(const rh_sim* s) {
+  if (s->shape_given || use_persist(s)) return s->ts;
+  const int64_t warps_per_sm = is_mixed(s) ? 4 : 12;
+  return s->sets[kNarrowSet].ntiles <= warps_per_sm * s->sm_count ? kNarrowSet : s->ts;
+}
+
 template <class R>
 StepArgs<R> make_args(rh_sim* s, const Lattice<R>& L, bool lattice_only) {
   StepArgs<R> a{};
   a.L = L;
-  a.cells = s->sets[s->ts].d_cells;
+  const rh_sim::TileSet& t = s->sets[active_set(s)];
+  a.cells = t.d_cells;
   a.dyn = s->d_dyn;
-  a.tiles = s->sets[s->ts].d_tiles;
+  a.tiles = t.d_tiles;
   a.partials = s->d_partials;
   a.out_wc = s->d_out_wc;
   a.out_ls = s->d_out_ls;
@@ -315,7 +343,7 @@ StepArgs<R> make_args(rh_sim* s, const Lattice<R>& L, bool lattice_only) {
 // One group's step: the tiles of cells [group_cell[g], group_cell[g+1]),
 // then the whole-cell update of those cells.
 cudaError_t launch_group(rh_sim* s, int g, bool out, bool lattice_only, cudaStream_t st) {
-  const rh_sim::TileSet& t = s->sets[s->ts];
+  const rh_sim::TileSet& t = s->sets[active_set(s)];
   const int c0 = s->group_cell[g], c1 = s->group_cell[g + 1];
   const int tb = t.hcells[c0].tile_begin;
   const int te = c1 < s->ncells ? t.hcells[c1].tile_begin : t.ntiles;
@@ -430,14 +458,6 @@ bool any_options(const rh_sim* s) {
 // sequence number and cell).
 size_t sync_bytes(int ncells) {
   return sizeof(CellSync) * (size_t)ncells + sizeof(unsigned int) * (2 + 4 * (size_t)ncells);
-}
-
-// Whether windows of steps run as one persistent launch: the run option, a
-// tile length the window kernel is compiled for, and a device that can
-// launch it cooperatively.
-bool use_persist(const rh_sim* s) {
-  const int tile = s->sets[s->ts].tile;
-  return s->opts.persistent && s->persist_ok && (tile == 64 || tile == 128);
 }
 
 // `n` steps of every cell as one persistent launch: the synchronisation
@@ -768,9 +788,9 @@ static int create_impl(rh_sim* s, const rh_cell_params* cells, int32_t ncells,
     s->hcells.push_back(cc);
   }
   int max_tiles = 0;
-  for (int k = 0; k < kNumTileSizes; ++k) {
+  for (int k = 0; k < kNumTileSets; ++k) {
     rh_sim::TileSet& t = s->sets[k];
-    t.tile = kTileSizes[k];
+    t.tile = tile_of_set(k);
     t.hcells = s->hcells;
     int nt = 0;
     for (int c = 0; c < ncells; ++c) {
@@ -790,6 +810,7 @@ static int create_impl(rh_sim* s, const rh_cell_params* cells, int32_t ncells,
     s->ts = -1;
     for (int k = 0; k < kNumTileSizes; ++k)
       if (kTileSizes[k] == want) s->ts = k;
+    s->shape_given = s->opts.block_size > 0;
     if (s->ts < 0) return fail(s, RH_ERR_ARG, "block_size %d is not a compiled tile length", want);
   }
   s->hcells = s->sets[s->ts].hcells;
@@ -800,6 +821,7 @@ static int create_impl(rh_sim* s, const rh_cell_params* cells, int32_t ncells,
   s->ls_rows_total = ls_off;
   s->device = s->opts.device;
   CK(cudaSetDevice(s->device));
+  CK(cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, s->device));
   CK(prepare_step_kernels());
   CK(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
   {
@@ -823,7 +845,7 @@ static int create_impl(rh_sim* s, const rh_cell_params* cells, int32_t ncells,
       s->maps_ok = s->maps_ok && build_stage_maps(s->Lf, s->stride, kTileSizes[k], s->maps[k]);
   }
   CK(cudaMalloc(&s->d_dyn, sizeof(CellDyn) * ncells));
-  for (int k = 0; k < kNumTileSizes; ++k) {
+  for (int k = 0; k < kNumTileSets; ++k) {
     rh_sim::TileSet& t = s->sets[k];
     CK(cudaMalloc(&t.d_cells, sizeof(CellConst) * ncells));
     CK(cudaMalloc(&t.d_tiles, sizeof(int4) * t.ntiles));
@@ -1111,7 +1133,7 @@ int rh_set_ap_clamp(rh_sim* s, int32_t cell, const double* v, int64_t n) {
   if (!s->d_apv[cell]) CK(cudaMalloc(&s->d_apv[cell], sizeof(double) * (size_t)n));
   CK(cudaMemcpy(s->d_apv[cell], v, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice));
   // every tile layout's copy of the cell constants points at the waveform
-  for (int k = 0; k < kNumTileSizes; ++k) {
+  for (int k = 0; k < kNumTileSets; ++k) {
     rh_sim::TileSet& t = s->sets[k];
     t.hcells[cell].apv = s->d_apv[cell];
     CK(cudaMemcpy(t.d_cells + cell, &t.hcells[cell], sizeof(CellConst), cudaMemcpyHostToDevice));
@@ -1656,6 +1678,8 @@ int rh_autotune(rh_sim* s, int32_t steps, int32_t* tile, double* ms_per_step) {
   const std::vector<double> t0 = s->t_host;
   const std::vector<char> a0 = s->active_host;
   const int ts0 = s->ts;
+  const bool given0 = s->shape_given;
+  s->shape_given = true;
   double best = 1e300;
   int best_k = ts0;
   cudaEvent_t e0, e1;
@@ -1708,6 +1732,7 @@ int rh_autotune(rh_sim* s, int32_t steps, int32_t* tile, double* ms_per_step) {
   s->t_host = t0;
   s->active_host = a0;
   s->ts = rc == RH_OK ? best_k : ts0;
+  s->shape_given = rc == RH_OK || given0;
   s->hcells = s->sets[s->ts].hcells;
   for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);
   s->graphs.clear();
@@ -1751,6 +1776,7 @@ int rh_set_launch_shape(rh_sim* s, const rh_launch_shape* shape) {
   CK(cudaSetDevice(s->device));
   CK(cudaStreamSynchronize(s->stream));
   s->ts = k;
+  s->shape_given = true;
   s->hcells = s->sets[k].hcells;
   s->opts.persistent = shape->persistent ? 1 : 0;
   s->fewer_ctas = shape->persistent && shape->fewer_ctas;
@@ -1870,6 +1896,7 @@ int rh_autotune_shapes(rh_sim* s, int32_t steps, rh_launch_shape* best,
           cand.push_back(rh_launch_shape{0, tile, 0, std::min(g, s->ncells), bulk});
   rh_launch_shape orig{};
   rh_get_launch_shape(s, &orig);
+  const bool given0 = s->shape_given;
   // save the state on the device; every candidate starts from it
   const size_t dyn_bytes = sizeof(CellDyn) * (size_t)s->ncells;
   void* backup = nullptr;
@@ -1937,6 +1964,7 @@ int rh_autotune_shapes(rh_sim* s, int32_t steps, rh_launch_shape* best,
   s->active_host = a0;
   if (ntried) *ntried = std::min(nt, max_tried);
   const int r = rh_set_launch_shape(s, rc == RH_OK ? &win : &orig);
+  if (rc != RH_OK) s->shape_given = given0;
   if (rc != RH_OK) return rc;
   if (r != RH_OK) return r;
   {

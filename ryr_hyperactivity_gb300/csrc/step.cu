@@ -193,6 +193,7 @@ cudaError_t launch_step(const StepArgs<R>& a, int ntiles, bool out, bool opt, in
   static const StageMaps kNoMaps{};
   const StageMaps& m = maps ? *maps : kNoMaps;
   switch (tile) {
+    case kNarrowTile: launch_bb<R, kNarrowTile, 0>(a, m, ntiles, out, opt, st); break;
     case 64: launch_b<R, 64>(a, m, ntiles, out, opt, staging, st); break;
     case 128: launch_b<R, 128>(a, m, ntiles, out, opt, staging, st); break;
     case 256: launch_b<R, 256>(a, m, ntiles, out, opt, staging, st); break;

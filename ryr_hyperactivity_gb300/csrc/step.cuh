@@ -13,6 +13,14 @@ constexpr int kNumTileSizes = 3;
 constexpr int kTileSizes[kNumTileSizes] = {64, 128, 256};
 constexpr int kDefaultTile = 128;
 
+// Narrow tiles, one warp per CTA, which the library uses by itself (they are
+// no launch shape) where the default tiles would leave SMs idle or unevenly
+// loaded; the simulator keeps their tile table after the kTileSizes ones.
+constexpr int kNarrowTile = 32;
+constexpr int kNarrowSet = kNumTileSizes;
+constexpr int kNumTileSets = kNumTileSizes + 1;
+constexpr int tile_of_set(int k) { return k == kNarrowSet ? kNarrowTile : kTileSizes[k]; }
+
 // Cell groups advanced on concurrent streams when the run options leave the
 // choice to the library.  Each group's step ends with its cell update, a
 // chain of dependent FP64 work that leaves most SMs to the other groups; with
@@ -26,8 +34,8 @@ constexpr int kDefaultGroups = 8;
 // so fewer, register-rich threads.
 template <class R, int B>
 __host__ __device__ constexpr int min_blocks_for() {
-  return sizeof(R) == 4 ? (B == 64 ? 10 : (B == 128 ? 5 : 2))
-                        : (B == 64 ? 6 : (B == 128 ? 3 : 1));
+  return sizeof(R) == 4 ? (B == 32 ? 20 : B == 64 ? 10 : (B == 128 ? 5 : 2))
+                        : (B == 32 ? 12 : B == 64 ? 6 : (B == 128 ? 3 : 1));
 }
 
 // Basal values of one cell (Init kernel, cuda_Cell_Detailed.cu:1121-1174),
@@ -86,7 +94,8 @@ cudaError_t launch_window(const StepArgs<R>& a, const WindowCtl& w, bool opt, in
 template <class R>
 cudaError_t window_grid(int tile, bool opt, bool fewer_ctas, int* ctas);
 
-// One time step with tiles of `tile` CRUs (one of kTileSizes).  `opt` selects
+// One time step with tiles of `tile` CRUs (one of kTileSizes, or kNarrowTile
+// with staging 0).  `opt` selects
 // the kernel variant that handles the per-cell build options of the lattice
 // update (perm, iso, slowncxchange, NCX form); without them a cell runs the
 // plain variant.
