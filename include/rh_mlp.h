@@ -55,35 +55,28 @@ int rh_mlp_last_error(const rh_mlp* m, char* buf, size_t n);
  *
  * d_params: device FP32 parameter vector in the layout above (what
  * rh_mlp_get_params returns); d_x: device [n x 4]; d_y: device [n x 3]; all
- * on the calling thread's current device.  Same kernels and the same result
+ * on the calling thread's current device.  Same kernel and the same result
  * as rh_mlp_forward with those parameters.  The work is queued on `stream`
  * (a cudaStream_t; NULL = the default stream) and the call returns without
  * waiting for it.
  *
- * The intermediate values live in one fixed device array inside the library,
- * RH_MLP_NOALLOC_SCRATCH_BYTES (4 MiB) per device, held from the library's
- * loading until process exit.  n above RH_MLP_NOALLOC_MAX_BATCH is rejected
- * with RH_ERR_ARG and a message in err (err may be NULL).  The first call on
- * a device looks up that array's device address (one-time set-up, repeated
- * when the call comes from another context of that device, e.g. after
- * cudaDeviceReset); make that first call before any stream capture.  All
- * calls on a device share the array: two calls whose work overlaps on the
- * GPU (different streams, or different threads without ordering) race and
- * give wrong results.  Each
- * call writes every scratch value it reads, so nothing left by an earlier
- * call reaches the result. */
-/* Check of the network's GEMM kernels (testing aid; synchronous, default
+ * The intermediate values live in the kernel's shared memory: the library
+ * keeps no array for them, and calls on different streams or threads are
+ * independent.  n above RH_MLP_NOALLOC_MAX_BATCH is rejected with RH_ERR_ARG
+ * and a message in err (err may be NULL). */
+/* Check of the library's GEMM kernels (testing aid; synchronous, default
  * stream): C[M x N] (FP32, row-major, leading dimension ldc) = sum over k of
  * A(m, k) B(k, n), with A(m, k) = A[m*sam + k*sak] and B(k, n) =
  * B[k*sbk + n*sbn] BF16 device arrays and C a device array; N <= 128.
- * tensor_cores = 1 runs the tcgen05 kernel (tensor-memory accumulator) the
- * network uses, 0 the mma.sync kernel kept as its independent check. */
+ * tensor_cores = 1 runs the tcgen05 kernel (tensor-memory accumulator; the
+ * general-stride form of the products in the network's own kernel), 0 the
+ * mma.sync kernel kept as its independent check. */
 int rh_mlp_gemm_check(const void* A, int32_t sam, int32_t sak, const void* B, int32_t sbk,
                       int32_t sbn, float* C, int32_t ldc, int32_t M, int32_t N, int32_t K,
                       int32_t tensor_cores);
 
 #define RH_MLP_NOALLOC_MAX_BATCH 4096
-#define RH_MLP_NOALLOC_SCRATCH_BYTES (4 * 1024 * 1024)
+#define RH_MLP_NOALLOC_SCRATCH_BYTES 0 /* device memory the library holds for it */
 int rh_mlp_forward_noalloc(const float* d_params, const float* d_x, int32_t n, float* d_y,
                            void* stream, char* err, size_t err_len);
 

@@ -5,11 +5,15 @@
 // mean), y2 = softplus(z2) (normalised APD90 variance).  Loss per sample:
 // BCE(y0, p) + (y1 - m)^2 + (y2 - s)^2, averaged over the batch.
 //
-// Every GEMM of the handle-based passes (forward Z = A W^T, backward
-// dA = dZ W and dW = dZ^T A) runs on Blackwell's 5th-generation tensor cores
-// through gemm_tc (tcgen05.mma, BF16 x BF16 -> FP32 accumulator in tensor
-// memory).  The no-allocation forward and the GEMM check keep gemm_bf16
-// (mma.sync m16n8k16), which also serves as gemm_tc's independent check.
+// One kernel, mlp_rows, runs a whole pass: each CTA keeps the network's
+// weights in shared memory and takes tiles of 128 samples through every layer
+// (and, in training, back through every layer and into the weight gradients)
+// with the products on Blackwell's 5th-generation tensor cores (tcgen05.mma,
+// BF16 x BF16 -> FP32 accumulators in tensor memory).  Nothing but inputs,
+// outputs and gradients touches global memory.  A second kernel,
+// mlp_finish, adds the CTAs' gradients in order and takes the Adam step.
+// gemm_tc and gemm_bf16 are general strided GEMMs on tcgen05 and mma.sync,
+// each other's check (rh_mlp_gemm_check).
 // Padded shapes: layer 1 K = 16 (4 inputs + zeros), layer 4 N = 8 (3
 // outputs + zeros; the tcgen05 MMA pads N to 16).
 #include <cuda.h>
@@ -22,9 +26,7 @@
 #include <string.h>
 
 #include <algorithm>
-#include <mutex>
 #include <string>
-#include <vector>
 
 #include "../../include/rh_mlp.h"
 
@@ -146,7 +148,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
 }  // namespace tc
 
 // C[M,N] (f32, row-major, ldc) = sum_k A(m,k) B(k,n) (+ C when accumulate),
-// with A and B addressed as in gemm_bf16; N <= 128.
+// with A and B addressed as in gemm_bf16; N <= 128.  The general form of the
+// products mlp_rows takes on its own tiles, reached through rh_mlp_gemm_check.
 __global__ void __launch_bounds__(128, 1)
     gemm_tc(const __nv_bfloat16* __restrict__ A, int sam, int sak,
             const __nv_bfloat16* __restrict__ Bm, int sbk, int sbn, float* C, int ldc, int M,
@@ -275,95 +278,525 @@ __global__ void __launch_bounds__(128, 1)
                  : "memory");
 }
 
-// Z += bias (per column); A = relu(Z) in BF16 (hidden layers).
-__global__ void bias_relu(float* Z, const float* bias, __nv_bfloat16* Aout, int M, int N) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (int64_t)M * N) return;
-  float z = Z[i] + bias[i % N];
-  Z[i] = z;
-  Aout[i] = __float2bfloat16(z > 0.f ? z : 0.f);
-}
-
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + expf(-x)); }
 __device__ __forceinline__ float softplusf_(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 
-// Output layer: y, loss terms and dZ4 (scaled by 1/B), in FP32 and BF16.
-__global__ void output_loss(float* Z4, const float* b4, const float* target, float* y,
-                            float* dz4, __nv_bfloat16* dz4b, float* loss_terms, int B) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= B) return;
-  float z0 = Z4[i * NOUT + 0] + b4[0], z1 = Z4[i * NOUT + 1] + b4[1], z2 = Z4[i * NOUT + 2] + b4[2];
-  float y0 = sigmoidf_(z0), y1 = z1, y2 = softplusf_(z2);
-  y[i * 3 + 0] = y0;
-  y[i * 3 + 1] = y1;
-  y[i * 3 + 2] = y2;
-  float l = 0.f;
-  float g0 = 0.f, g1 = 0.f, g2 = 0.f;
-  if (target) {
-    const float p = target[i * 3 + 0], m = target[i * 3 + 1], s = target[i * 3 + 2];
-    const float e = 1e-7f;
-    l = -(p * logf(fmaxf(y0, e)) + (1.f - p) * logf(fmaxf(1.f - y0, e))) + (y1 - m) * (y1 - m) +
-        (y2 - s) * (y2 - s);
-    const float invB = 1.f / (float)B;
-    g0 = (y0 - p) * invB;
-    g1 = 2.f * (y1 - m) * invB;
-    g2 = 2.f * (y2 - s) * sigmoidf_(z2) * invB;
-    loss_terms[i] = l;
+// ---- the parameter vector (rh_mlp.h) and its BF16 image ----
+constexpr int kW1 = 0, kB1 = kW1 + H * KIN, kW2 = kB1 + H, kB2 = kW2 + H * H, kW3 = kB2 + H,
+              kB3 = kW3 + H * H, kW4 = kB3 + H, kB4 = kW4 + NOUT * H, kNPar = kB4 + NOUT;
+constexpr int NPAD = 16;  // output rows of the MMA
+// The image holds the four weight matrices as the MMA's operands: element
+// (row, k) of a matrix of `rows` rows at tc::core_off(row, k, rows), so that
+// a CTA's copy is one contiguous bulk copy.
+constexpr int kImg1 = 0, kImg2 = kImg1 + H * KIN * 2, kImg3 = kImg2 + H * H * 2,
+              kImg4 = kImg3 + H * H * 2, kImgBytes = kImg4 + NPAD * H * 2;
+
+// Layer of parameter i, and for a weight its row, column and image offset.
+struct ParamPlace {
+  int img;      // byte offset in the image, -1 for a bias
+  bool padded;  // a padding weight: always zero
+};
+__device__ __forceinline__ ParamPlace place_of(int i) {
+  if (i < kB1) {
+    const int r = i / KIN, k = i % KIN;
+    return {kImg1 + (int)tc::core_off(r, k, H), k >= RH_MLP_IN};
   }
-  const float gg[NOUT] = {g0, g1, g2, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int q = 0; q < NOUT; ++q) {
-    dz4[i * NOUT + q] = gg[q];
-    dz4b[i * NOUT + q] = __float2bfloat16(gg[q]);
+  if (i >= kW2 && i < kB2) {
+    const int j = i - kW2;
+    return {kImg2 + (int)tc::core_off(j / H, j % H, H), false};
+  }
+  if (i >= kW3 && i < kB3) {
+    const int j = i - kW3;
+    return {kImg3 + (int)tc::core_off(j / H, j % H, H), false};
+  }
+  if (i >= kW4 && i < kB4) {
+    const int j = i - kW4;
+    return {kImg4 + (int)tc::core_off(j / H, j % H, NPAD), j / H >= RH_MLP_OUT};
+  }
+  return {-1, false};
+}
+
+constexpr int kRowThreads = 512;  // of a mlp_rows CTA
+
+// ---- shared memory of mlp_rows ----
+struct RowsSmem {
+  static constexpr int kW = 0;                       // the image
+  static constexpr int kX0 = kW + kImgBytes;         // packed inputs, 128 x 16
+  static constexpr int kA = kX0 + 128 * KIN * 2;     // activations, 128 x 128 each
+  static constexpr int kTile = 128 * H * 2;
+  // forward only: one activation tile, overwritten layer by layer
+  static constexpr int kBiasF = kA + kTile;
+  // training: three activation tiles, the dZ tile, dZ4, the column sums
+  static constexpr int kD = kA + 3 * kTile;
+  static constexpr int kD4 = kD + kTile;
+  static constexpr int kRed = kD4 + 128 * NPAD * 2;  // float[3][4][128]
+  static constexpr int kBiasT = kRed + 3 * 4 * H * 4;
+  static constexpr int kBiasBytes = (3 * H + NOUT) * 4;
+  static constexpr int bytes(bool train) { return (train ? kBiasT : kBiasF) + kBiasBytes; }
+};
+static_assert(RowsSmem::bytes(true) <= 227 * 1024, "shared memory of a CTA");
+
+struct RowsArgs {
+  const unsigned char* img;  // BF16 image; nullptr: converted from params in the kernel
+  const float* params;       // FP32 vector
+  const float* x;            // n x 4
+  const float* target;       // n x 3 (training)
+  float* y;                  // n x 3 (forward)
+  float* loss;               // n loss terms (training)
+  float* part;               // [gridDim.x][kNPar] gradients (training)
+  int n;
+  int* err;                  // set when a wait gave up; nullptr: y becomes NaN
+};
+
+// One MMA chain: K = 16 ksteps, descriptors advancing by da and db bytes.
+__device__ __forceinline__ void mma_chain(uint32_t acc, uint32_t a, uint32_t a_lbo, uint32_t a_sbo,
+                                          uint32_t da, uint32_t b, uint32_t b_lbo, uint32_t b_sbo,
+                                          uint32_t db, uint32_t idesc, int ksteps, bool add) {
+  for (int s = 0; s < ksteps; ++s) {
+    const uint64_t ad = tc::smem_desc(a + s * da, a_lbo, a_sbo);
+    const uint64_t bd = tc::smem_desc(b + s * db, b_lbo, b_sbo);
+    const uint32_t on = (add || s > 0) ? 1u : 0u;
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(acc),
+        "l"(ad), "l"(bd), "r"(idesc), "r"(on)
+        : "memory");
   }
 }
 
-// dZ = dA * relu'(Z) -> BF16
-__global__ void relu_backward(const float* dA, const float* Z, __nv_bfloat16* dZb, float* dZf,
-                              int64_t n) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float d = Z[i] > 0.f ? dA[i] : 0.f;
-  dZf[i] = d;
-  dZb[i] = __float2bfloat16(d);
+__device__ __forceinline__ void tmem_load32(uint32_t addr, uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
+      "%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+        "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
+        "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
+        "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      : "r"(addr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_load8(uint32_t addr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]),
+                 "=r"(v[6]), "=r"(v[7])
+               : "r"(addr)
+               : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// db[n] = sum over rows of dZ (fixed order per column)
-__global__ void bias_grad(const float* dZ, float* db, int M, int N) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  float s = 0.f;
-  for (int m = 0; m < M; ++m) s += dZ[(int64_t)m * N + n];
-  db[n] = s;
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  return (uint32_t)__bfloat16_as_ushort(__float2bfloat16(lo)) |
+         ((uint32_t)__bfloat16_as_ushort(__float2bfloat16(hi)) << 16);
 }
 
-// Adam step on FP32 masters, refresh the BF16 copies.  Padded entries (mask
-// 0) stay zero.
-__global__ void adam_update(float* w, const float* g, float* m, float* v, __nv_bfloat16* wb,
-                            const float* mask, int n, float lr, float b1, float b2, float eps,
-                            float bc1, float bc2) {
+// 32 values of one row, columns col.., to BF16 in an operand tile of 128 rows.
+__device__ __forceinline__ void store_row32(unsigned char* tile, int row, int col,
+                                            const float (&v)[32]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint4 w;
+    w.x = pack_bf16(v[8 * q], v[8 * q + 1]);
+    w.y = pack_bf16(v[8 * q + 2], v[8 * q + 3]);
+    w.z = pack_bf16(v[8 * q + 4], v[8 * q + 5]);
+    w.w = pack_bf16(v[8 * q + 6], v[8 * q + 7]);
+    *reinterpret_cast<uint4*>(tile + tc::core_off(row, col + 8 * q, 128)) = w;
+  }
+}
+
+// Sum over the warp's lanes of each of 32 values: lane i returns the sum of
+// v[i] (a halving exchange, 31 shuffles).
+__device__ __forceinline__ float column_sums(float (&v)[32], int lane) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int i = 0; i < off; ++i) {
+      const float give = up ? v[i] : v[i + off];
+      const float keep = up ? v[i + off] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+    }
+  }
+  return v[0];
+}
+
+// The caller's FP32 weights as the BF16 image (what mlp_load writes), eight
+// weights of a row at a time; a warp takes 16 rows of two neighbouring groups
+// of eight, whose loads fill 64-byte segments and whose stores conflict twice.
+__device__ __forceinline__ void image_from_params(const float* params, unsigned char* img,
+                                                  int tid) {
+  const bool aligned = (reinterpret_cast<uintptr_t>(params) & 15) == 0;
+  for (int i = tid; i < kImgBytes / 16; i += kRowThreads) {
+    int row, k, src, rows = H, rvalid = H, kvalid = H, base;
+    if (i < kImg2 / 16) {
+      row = i >> 1;
+      k = (i & 1) * 8;
+      src = kW1 + row * KIN + k;
+      kvalid = RH_MLP_IN;
+      base = kImg1;
+    } else if (i < kImg4 / 16) {
+      const int j = (i - kImg2 / 16) & 2047, l = (i - kImg2 / 16) >> 11;
+      row = ((j >> 1) & 15) | ((j >> 8) << 4);
+      k = ((j & 1) | (((j >> 5) & 7) << 1)) * 8;
+      src = (l == 0 ? kW2 : kW3) + row * H + k;
+      base = l == 0 ? kImg2 : kImg3;
+    } else {
+      const int j = i - kImg4 / 16;
+      row = j >> 4;
+      k = (j & 15) * 8;
+      src = kW4 + row * H + k;
+      rows = NPAD;
+      rvalid = RH_MLP_OUT;
+      base = kImg4;
+    }
+    float v[8];
+    if (row >= rvalid) {  // padding rows; those past the vector's are not read
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = 0.f;
+    } else if (aligned) {
+      const float4 lo = *reinterpret_cast<const float4*>(params + src);
+      const float4 hi = *reinterpret_cast<const float4*>(params + src + 4);
+      v[0] = lo.x, v[1] = lo.y, v[2] = lo.z, v[3] = lo.w;
+      v[4] = hi.x, v[5] = hi.y, v[6] = hi.z, v[7] = hi.w;
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = params[src + q];
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (k + q >= kvalid) v[q] = 0.f;
+    *reinterpret_cast<uint4*>(img + base + tc::core_off(row, k, rows)) =
+        make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]),
+                   pack_bf16(v[6], v[7]));
+  }
+}
+
+// The network on tiles of 128 samples: CTA c takes tiles c, c + gridDim.x, ...
+// with 512 threads; thread (row, quarter) owns one sample (a tensor-memory
+// lane) and 32 of its 128 columns.
+//
+// What bounds it: a tile's arithmetic is a few microseconds of one SM's tensor
+// cores, so a pass is the latency of its layers, one after the other: an MMA
+// chain, a round trip to an mbarrier and an epilogue each (10 us forward, 13 us
+// a tile in training, plus 12 us for the weights and the gradients).  So the
+// layers run in one CTA with the activations in shared memory.  One launch per
+// product, bias and activation, as before, cost 24 us of strided staging per
+// product (500 us for a dW over 4,096 samples in one CTA) and ten to 25
+// launches.  Whole calls, before and now: 65,536 predictions 2.20 ms and 95 us,
+// an epoch of twelve 256-sample steps 5.50 and 0.86 ms, gradients of 4,096
+// samples 2.04 ms and 58 us, the no-allocation forward of 1,000 samples 61 and
+// 12 us.  256 threads (64 columns each) were slower: 44 us against 38 for two
+// training tiles.
+//
+// Operands: every tile in shared memory is the no-swizzle core-matrix layout
+// of 8 rows x 16 bytes, rows along samples (or output units).  Read K-major it
+// is the forward operand (samples x features); the same bytes read MN-major
+// (the instruction descriptor's transpose bits, with the two strides
+// exchanged) are the transposed operands of dW = dZ^T A and dA = dZ W, so
+// nothing is transposed or stored twice.
+template <bool TRAIN>
+__global__ void __launch_bounds__(kRowThreads, 1) mlp_rows(const RowsArgs a) {
+  extern __shared__ __align__(128) unsigned char sm[];
+  __shared__ __align__(8) uint64_t bars[2];  // MMAs done; weights landed
+  __shared__ uint32_t tmem_base;
+  using S = RowsSmem;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int quarter = warp >> 2, row = (warp & 3) * 32 + lane, col = quarter * 32;
+  float* bias = reinterpret_cast<float*>(sm + (TRAIN ? S::kBiasT : S::kBiasF));
+  constexpr uint32_t kCols = TRAIN ? 512u : 128u;
+  const uint32_t mma_bar = tc::saddr(&bars[0]), w_bar = tc::saddr(&bars[1]);
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mma_bar) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(w_bar) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (a.img) {
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(w_bar),
+                   "r"((uint32_t)kImgBytes)
+                   : "memory");
+      asm volatile(
+          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
+              "r"(tc::saddr(sm + S::kW)),
+          "l"(a.img), "r"((uint32_t)kImgBytes), "r"(w_bar)
+          : "memory");
+    }
+  }
+  __syncwarp();
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     tc::saddr(&tmem_base)),
+                 "r"(kCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  for (int i = tid; i < 3 * H + NOUT; i += kRowThreads) {
+    const int l = i / H, j = i % H;
+    bias[i] = a.params[(l == 0 ? kB1 : l == 1 ? kB2 : l == 2 ? kB3 : kB4) + j];
+  }
+  if (!a.img) image_from_params(a.params, sm + S::kW, tid);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_base;
+  const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  bool ok = !a.img || tc::mbar_wait(w_bar, 0);
+  // accumulators in tensor memory: the layer's product, then (training) dW2,
+  // dW3, dW1 and dW4 (transposed: 128 inputs x 16 outputs)
+  constexpr uint32_t kDW2 = 128, kDW3 = 256, kDW1 = 384, kDW4 = 400;
+  constexpr uint32_t kTA = 1u << 15, kTB = 1u << 16;  // MN-major A, B
+  const uint32_t id128 = tc::instr_desc(128, H), id16 = tc::instr_desc(128, NPAD);
+  const uint32_t sw = tc::saddr(sm + S::kW), sx = tc::saddr(sm + S::kX0);
+  const uint32_t w1 = sw + kImg1, w2 = sw + kImg2, w3 = sw + kImg3, w4 = sw + kImg4;
+  // K-major operand of 128 rows: lbo 2048 (next 8 of K), sbo 128 (next 8
+  // rows), 4096 a K step; MN-major: lbo 128, sbo 2048, 256 a K step
+  constexpr uint32_t kL = 2048, kS = 128, kStep = 4096, kStepT = 256;
+  uint32_t phase = 0;
+  // makes the CTA's shared-memory writes visible to the tensor cores, then
+  // thread 0 issues `mmas` and every thread waits for them; false (in every
+  // thread, before any MMA of this call) once a wait has given up
+  auto run_mmas = [&](auto mmas) -> bool {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (!__syncthreads_and(ok ? 1 : 0)) return false;
+    if (tid == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      mmas();
+      asm volatile(
+          "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+              mma_bar)
+          : "memory");
+    }
+    ok = tc::mbar_wait(mma_bar, phase);
+    phase ^= 1u;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    return true;
+  };
+  const bool x16 = (reinterpret_cast<uintptr_t>(a.x) & 15) == 0;
+  const float inv_n = 1.f / (float)a.n;
+  float db[4] = {0.f, 0.f, 0.f, 0.f};  // thread j < 128: column j of db1..3; db4 of thread j < 3
+  const int tiles = (a.n + 127) / 128;
+  bool first = true;
+  auto one_tile = [&](int t) -> bool {
+    const int r = t * 128 + row;
+    const bool valid = r < a.n;
+    if (quarter == 0) {  // inputs to BF16, zero-padded to 16
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (valid) {
+        if (x16) {
+          x = reinterpret_cast<const float4*>(a.x)[r];
+        } else {
+          const float* p = a.x + (size_t)r * RH_MLP_IN;
+          x = make_float4(p[0], p[1], p[2], p[3]);
+        }
+      }
+      const uint4 w = make_uint4(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w), 0u, 0u);
+      *reinterpret_cast<uint4*>(sm + S::kX0 + tc::core_off(row, 0, 128)) = w;
+      *reinterpret_cast<uint4*>(sm + S::kX0 + tc::core_off(row, 8, 128)) = make_uint4(0, 0, 0, 0);
+    }
+    uint32_t mask[3];  // z > 0 of this thread's columns
+#pragma unroll
+    for (int l = 0; l < 3; ++l) {
+      unsigned char* out = sm + S::kA + (TRAIN ? l : 0) * S::kTile;
+      const uint32_t in = l == 0 ? sx : tc::saddr(sm + S::kA + (TRAIN ? l - 1 : 0) * S::kTile);
+      const uint32_t w = l == 0 ? w1 : l == 1 ? w2 : w3;
+      if (!run_mmas([&] {
+            mma_chain(tmem, in, kL, kS, kStep, w, kL, kS, kStep, id128, l == 0 ? 1 : H / 16, false);
+          }))
+        return false;
+      uint32_t raw[32];
+      tmem_load32(lanes + col, raw);
+      float v[32];
+      uint32_t m = 0u;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const float z = __uint_as_float(raw[j]) + bias[l * H + col + j];
+        if (z > 0.f) m |= 1u << j;
+        v[j] = z > 0.f ? z : 0.f;
+      }
+      mask[l] = m;
+      store_row32(out, row, col, v);
+    }
+    // output layer
+    const uint32_t a3 = tc::saddr(sm + S::kA + (TRAIN ? 2 : 0) * S::kTile);
+    if (!run_mmas([&] {
+          mma_chain(tmem, a3, kL, kS, kStep, w4, 256, kS, 512, id16, H / 16, false);
+        }))
+      return false;
+    if (quarter == 0) {
+      uint32_t raw[8];
+      tmem_load8(lanes, raw);
+      const float* b4 = bias + 3 * H;
+      const float z0 = __uint_as_float(raw[0]) + b4[0], z1 = __uint_as_float(raw[1]) + b4[1],
+                  z2 = __uint_as_float(raw[2]) + b4[2];
+      const float y0 = sigmoidf_(z0), y1 = z1, y2 = softplusf_(z2);
+      if constexpr (!TRAIN) {
+        if (valid && ok) {
+          float* y = a.y + (size_t)r * RH_MLP_OUT;
+          y[0] = y0;
+          y[1] = y1;
+          y[2] = y2;
+        }
+      } else {
+        float g0 = 0.f, g1 = 0.f, g2 = 0.f;  // dZ4, scaled by 1/n
+        if (valid) {
+          const float* tg = a.target + (size_t)r * RH_MLP_OUT;
+          const float p = tg[0], m = tg[1], s = tg[2];
+          const float e = 1e-7f;
+          a.loss[r] = -(p * logf(fmaxf(y0, e)) + (1.f - p) * logf(fmaxf(1.f - y0, e))) +
+                      (y1 - m) * (y1 - m) + (y2 - s) * (y2 - s);
+          g0 = (y0 - p) * inv_n;
+          g1 = 2.f * (y1 - m) * inv_n;
+          g2 = 2.f * (y2 - s) * sigmoidf_(z2) * inv_n;
+        }
+        const uint4 w = make_uint4(pack_bf16(g0, g1), pack_bf16(g2, 0.f), 0u, 0u);
+        *reinterpret_cast<uint4*>(sm + S::kD4 + tc::core_off(row, 0, 128)) = w;
+        *reinterpret_cast<uint4*>(sm + S::kD4 + tc::core_off(row, 8, 128)) =
+            make_uint4(0, 0, 0, 0);
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = j == 0 ? g0 : j == 1 ? g1 : j == 2 ? g2 : 0.f;
+        const float s = column_sums(v, lane);
+        db[3] += s;  // lane j < 3 of each of the four row groups; added up at the end
+      }
+    }
+    if constexpr (TRAIN) {
+      float* red = reinterpret_cast<float*>(sm + S::kRed);
+      const uint32_t d4 = tc::saddr(sm + S::kD4), dd = tc::saddr(sm + S::kD);
+      const uint32_t act[3] = {tc::saddr(sm + S::kA), tc::saddr(sm + S::kA + S::kTile),
+                               tc::saddr(sm + S::kA + 2 * S::kTile)};
+#pragma unroll
+      for (int l = 2; l >= 0; --l) {
+        // dW of the layer above (over the tile's 128 samples) and dA of this one
+        if (!run_mmas([&] {
+              if (l == 2) {
+                mma_chain(tmem + kDW4, act[2], kS, kL, kStepT, d4, kS, kL, kStepT, id16 | kTA | kTB,
+                          8, !first);
+                mma_chain(tmem, d4, kL, kS, 0, w4, kS, 256, 0, id128 | kTB, 1, false);
+              } else {
+                mma_chain(tmem + (l == 1 ? kDW3 : kDW2), dd, kS, kL, kStepT, act[l], kS, kL, kStepT,
+                          id128 | kTA | kTB, 8, !first);
+                mma_chain(tmem, dd, kL, kS, kStep, l == 1 ? w3 : w2, kS, kL, kStepT, id128 | kTB, 8,
+                          false);
+              }
+            }))
+          return false;
+        uint32_t raw[32];
+        tmem_load32(lanes + col, raw);
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = (mask[l] >> j & 1u) ? __uint_as_float(raw[j]) : 0.f;
+        store_row32(sm + S::kD, row, col, v);
+        red[(l * 4 + (warp & 3)) * H + col + lane] = column_sums(v, lane);
+      }
+      if (!run_mmas([&] {
+            mma_chain(tmem + kDW1, dd, kS, kL, kStepT, sx, kS, kL, kStepT, id16 | kTA | kTB, 8,
+                      !first);
+          }))
+        return false;
+      if (tid < H) {
+#pragma unroll
+        for (int l = 0; l < 3; ++l)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) db[l] += red[(l * 4 + q) * H + tid];
+      }
+      first = false;
+    }
+    return true;
+  };
+  bool done = true;
+  for (int t = blockIdx.x; t < tiles && done; t += gridDim.x) done = one_tile(t);
+  done = __syncthreads_and((done && ok) ? 1 : 0) != 0;
+  if (!done) {
+    if (tid == 0 && a.err) *a.err = 1;  // host memory, read after a synchronisation
+    if (!TRAIN && !a.err)
+      for (int t = blockIdx.x; t < tiles; t += gridDim.x)
+        for (int i = tid; i < 128 * RH_MLP_OUT; i += kRowThreads)
+          if (t * 128 + i / RH_MLP_OUT < a.n)
+            a.y[(size_t)t * 128 * RH_MLP_OUT + i] = __int_as_float(0x7fc00000);
+  } else if constexpr (TRAIN) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    float* g = a.part + (size_t)blockIdx.x * kNPar;
+    // the lower two quarters write dW2 and dW1, the upper two dW3 and dW4
+    // (64 columns of a thread's accumulator row each)
+    const bool lower = quarter < 2;
+    const int c0 = (quarter & 1) * 64;
+    float* gw = g + (lower ? kW2 : kW3) + row * H + c0;
+#pragma unroll 1
+    for (int c = 0; c < 64; c += 32) {
+      uint32_t raw[32];
+      tmem_load32(lanes + (lower ? kDW2 : kDW3) + c0 + c, raw);
+#pragma unroll
+      for (int j = 0; j < 32; j += 4)  // parameter offsets are multiples of 4
+        *reinterpret_cast<uint4*>(gw + c + j) =
+            make_uint4(raw[j], raw[j + 1], raw[j + 2], raw[j + 3]);
+    }
+    {
+      uint32_t raw[8];
+      if (lower) {  // 8 of the 16 input columns
+        const int q = quarter * 8;
+        tmem_load8(lanes + kDW1 + q, raw);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) g[kW1 + row * KIN + q + j] = __uint_as_float(raw[j]);
+      } else if (quarter == 2) {
+        tmem_load8(lanes + kDW4, raw);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) g[kW4 + j * H + row] = __uint_as_float(raw[j]);
+      }
+    }
+    if (tid < H) {
+      g[kB1 + tid] = db[0];
+      g[kB2 + tid] = db[1];
+      g[kB3 + tid] = db[2];
+    }
+    float* red = reinterpret_cast<float*>(sm + S::kRed);
+    __syncthreads();  // the sums of the last tile have been read
+    if (quarter == 0 && lane < NOUT) red[(warp & 3) * NOUT + lane] = db[3];
+    __syncthreads();
+    if (tid < NOUT)
+      g[kB4 + tid] = red[tid] + red[NOUT + tid] + red[2 * NOUT + tid] + red[3 * NOUT + tid];
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  __syncwarp();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols)
+                 : "memory");
+}
+
+// What follows a training pass: the CTAs' gradients added in order, then
+// either written out or taken as one Adam step on the FP32 master weights,
+// refreshing the BF16 image.  Padding weights stay zero.
+struct AdamStep {
+  float lr, b1, b2, eps, bc1, bc2;
+};
+__global__ void mlp_finish(const float* part, int nparts, float* grads, float* w, float* m, float* v,
+                           unsigned char* img, AdamStep s) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (mask && mask[i] == 0.f) {
-    w[i] = 0.f;
-    if (wb) wb[i] = __float2bfloat16(0.f);
+  if (i >= kNPar) return;
+  float gi = 0.f;
+  for (int c = 0; c < nparts; ++c) gi += part[(size_t)c * kNPar + i];
+  if (grads) {
+    grads[i] = gi;
     return;
   }
-  float gi = g[i];
-  float mi = b1 * m[i] + (1.f - b1) * gi;
-  float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+  const ParamPlace p = place_of(i);
+  if (p.padded) return;
+  const float mi = s.b1 * m[i] + (1.f - s.b1) * gi;
+  const float vi = s.b2 * v[i] + (1.f - s.b2) * gi * gi;
   m[i] = mi;
   v[i] = vi;
-  float wi = w[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+  const float wi = w[i] - s.lr * (mi / s.bc1) / (sqrtf(vi / s.bc2) + s.eps);
   w[i] = wi;
-  if (wb) wb[i] = __float2bfloat16(wi);
+  if (p.img >= 0) *reinterpret_cast<__nv_bfloat16*>(img + p.img) = __float2bfloat16(wi);
 }
 
-// inputs (B x 4 floats) -> padded BF16 rows of 16
-__global__ void pack_inputs(const float* x, __nv_bfloat16* X0, int B) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (int64_t)B * KIN) return;
-  const int r = (int)(i / KIN), c = (int)(i % KIN);
-  X0[i] = __float2bfloat16(c < RH_MLP_IN ? x[r * RH_MLP_IN + c] : 0.f);
+// New parameters in w: padding weights to zero, the BF16 image refreshed.
+__global__ void mlp_load(float* w, unsigned char* img) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= kNPar) return;
+  const ParamPlace p = place_of(i);
+  if (p.padded) w[i] = 0.f;
+  if (p.img >= 0) *reinterpret_cast<__nv_bfloat16*>(img + p.img) = __float2bfloat16(w[i]);
 }
 
 unsigned blocks(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -372,20 +805,27 @@ unsigned blocks(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 // ---------------------------------------------------------------- host side
 
+constexpr int kChunk = 16384;    // samples of one forward launch
+constexpr int kMaxParts = 152;   // CTAs of a training pass
+
 struct rh_mlp {
   int bmax = 0;
+  int device = 0;
   cudaStream_t st = nullptr;
-  // parameters: FP32 masters, BF16 copies, Adam moments, gradients
-  float* P = nullptr;  // all FP32 buffers in one allocation
-  __nv_bfloat16* Pb = nullptr;
-  float *w[4], *b[4], *gw[4], *gb[4], *mw[4], *vw[4], *mb[4], *vb[4], *maskw[4];
-  __nv_bfloat16* wb[4];
-  int wn[4], wk[4];
-  // activations
-  __nv_bfloat16 *X0, *A[3], *dZb[4];
-  float *Z[4], *dA, *dZf, *y, *target, *xin, *loss;
+  float* P = nullptr;            // w, m, v, then the CTAs' gradients
+  float *w = nullptr, *m = nullptr, *v = nullptr, *part = nullptr;
+  unsigned char* img = nullptr;  // BF16 weights (kImgBytes)
+  // Host memory the kernels read and write directly (pinned, mapped): inputs
+  // of two chunks and targets of a batch (where the device cannot read the
+  // caller's own memory), outputs of two chunks or loss terms, gradients, the
+  // error flag.
+  unsigned char* host = nullptr;
+  float *h_x = nullptr, *h_t = nullptr, *h_out = nullptr, *h_g = nullptr;
+  int* h_err = nullptr;          // set by a pass whose wait gave up
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  bool direct = false;  // kernels can read pageable host memory (hardware page tables)
+  int chunk = 0;        // samples of one forward launch
   int64_t step = 0;
-  int* gemm_err = nullptr;  // set by a tcgen05 GEMM whose wait gave up
   std::string err;
 };
 
@@ -402,86 +842,52 @@ int ck(rh_mlp* m, cudaError_t e, const char* what) {
     if (r_) return r_;                         \
   } while (0)
 
-// Every GEMM of the network's handle-based passes runs on the tcgen05
-// kernel (the no-allocation forward keeps the mma.sync kernel).
-int gemm(rh_mlp* m, const __nv_bfloat16* A, int sam, int sak, const __nv_bfloat16* B, int sbk,
-         int sbn, float* C, int ldc, int M, int N, int K, int acc) {
-  gemm_tc<<<(M + tc::kM - 1) / tc::kM, 128, tc::kSmemA + tc::kSmemB, m->st>>>(
-      A, sam, sak, B, sbk, sbn, C, ldc, M, N, K, acc, m->gemm_err);
-  return ck(m, cudaGetLastError(), "gemm");
-}
-
-// After a stream synchronisation: RH_ERR_TIMEOUT when a GEMM's wait gave up.
-int check_gemm(rh_mlp* m) {
-  int h = 0;
-  MCK(cudaMemcpy(&h, m->gemm_err, sizeof(int), cudaMemcpyDeviceToHost));
-  if (h) {
-    cudaMemset(m->gemm_err, 0, sizeof(int));
-    m->err = "a tensor-core GEMM's wait for its MMAs ran out";
+// After a stream synchronisation: RH_ERR_TIMEOUT when a pass's wait gave up.
+int check_wait(rh_mlp* m) {
+  if (*m->h_err) {
+    *m->h_err = 0;
+    m->err = "a wait for the tensor cores ran out";
     return RH_ERR_TIMEOUT;
   }
   return RH_OK;
 }
 
-int forward(rh_mlp* m, int B) {
-  // layer l: Z = A_{l-1} W_l^T  (W_l stored n x k, row-major)
-  const __nv_bfloat16* in = m->X0;
-  int kin = KIN;
-  for (int l = 0; l < 3; ++l) {
-    int r = gemm(m, in, kin, 1, m->wb[l], 1, kin, m->Z[l], H, B, H, kin, 0);
-    if (r) return r;
-    bias_relu<<<blocks((int64_t)B * H, 256), 256, 0, m->st>>>(m->Z[l], m->b[l], m->A[l], B, H);
-    in = m->A[l];
-    kin = H;
-  }
-  return gemm(m, m->A[2], H, 1, m->wb[3], 1, H, m->Z[3], NOUT, B, NOUT, H, 0);
+// Where the kernels read `count` floats of the caller's `p`: in place, or
+// from a copy in `stage`.  In place is as fast or faster (a 65,536-point sweep
+// 95 against 130 us, gradients of 4,096 samples 58 against 64, a 256-sample
+// step 70 either way).
+const float* reachable(const rh_mlp* m, const float* p, size_t count, float* stage) {
+  if (m->direct) return p;
+  memcpy(stage, p, count * sizeof(float));
+  return stage;
 }
 
-int backward(rh_mlp* m, int B) {
-  // output layer gradients were written by output_loss into dZf/dZb[3]
-  // dW4 = dZ4^T A3 ; db4 = sum dZ4 ; dA3 = dZ4 W4
-  int r;
-  const __nv_bfloat16* acts[4] = {m->X0, m->A[0], m->A[1], m->A[2]};
-  const int kins[4] = {KIN, H, H, H};
-  const int nouts[4] = {H, H, H, NOUT};
-  for (int l = 3; l >= 0; --l) {
-    const int N = nouts[l], K = kins[l];
-    // dW_l (N x K) = dZ_l^T (N x B) * A_{l-1} (B x K)
-    if ((r = gemm(m, m->dZb[l], 1, N, acts[l], K, 1, m->gw[l], K, N, K, B, 0))) return r;
-    if (l == 3) {
-      // dZ4 in FP32 lives in dA's first B*8 entries (written by output_loss)
-      bias_grad<<<blocks(N, 128), 128, 0, m->st>>>(m->dA, m->gb[l], B, N);
-    } else {
-      bias_grad<<<blocks(N, 128), 128, 0, m->st>>>(m->dZf, m->gb[l], B, N);
-    }
-    if (l == 0) break;
-    // dA_{l-1} (B x K) = dZ_l (B x N) * W_l (N x K)
-    if ((r = gemm(m, m->dZb[l], N, 1, m->wb[l], K, 1, m->dA, K, B, K, N, 0))) return r;
-    relu_backward<<<blocks((int64_t)B * K, 256), 256, 0, m->st>>>(m->dA, m->Z[l - 1], m->dZb[l - 1],
-                                                                m->dZf, (int64_t)B * K);
-  }
-  return ck(m, cudaGetLastError(), "backward");
+// One training pass: loss terms to h_out, each CTA's gradients to part.  A
+// batch of up to two tiles is one CTA's work, whose accumulators then hold
+// the whole batch's sums; a larger one is spread a tile to a CTA, and the
+// short accumulations and the ordered FP32 sum of the CTAs' gradients are more
+// exact than one accumulator over the batch (4,096 samples: median error
+// 8e-8 relative against 2e-6).
+int train_pass(rh_mlp* m, const float* x, const float* target, int n, int* nparts) {
+  const int tiles = (n + 127) / 128;
+  *nparts = tiles <= 2 ? 1 : std::min(tiles, kMaxParts);
+  RowsArgs a{};
+  a.img = m->img;
+  a.params = m->w;
+  a.x = reachable(m, x, (size_t)n * RH_MLP_IN, m->h_x);
+  a.target = reachable(m, target, (size_t)n * RH_MLP_OUT, m->h_t);
+  a.loss = m->h_out;
+  a.part = m->part;
+  a.n = n;
+  a.err = m->h_err;
+  mlp_rows<true><<<*nparts, kRowThreads, RowsSmem::bytes(true), m->st>>>(a);
+  return ck(m, cudaGetLastError(), "training pass");
 }
 
-int run_loss(rh_mlp* m, int B, const float* xh, const float* th, float* loss_out) {
-  MCK(cudaMemcpyAsync(m->xin, xh, sizeof(float) * RH_MLP_IN * B, cudaMemcpyHostToDevice, m->st));
-  if (th)
-    MCK(cudaMemcpyAsync(m->target, th, sizeof(float) * 3 * B, cudaMemcpyHostToDevice, m->st));
-  pack_inputs<<<blocks((int64_t)B * KIN, 256), 256, 0, m->st>>>(m->xin, m->X0, B);
-  int r = forward(m, B);
-  if (r) return r;
-  output_loss<<<blocks(B, 128), 128, 0, m->st>>>(m->Z[3], m->b[3], th ? m->target : nullptr, m->y,
-                                                 m->dA, m->dZb[3], m->loss, B);
-  MCK(cudaGetLastError());
-  if (loss_out && th) {
-    std::vector<float> l(B);
-    MCK(cudaMemcpyAsync(l.data(), m->loss, sizeof(float) * B, cudaMemcpyDeviceToHost, m->st));
-    MCK(cudaStreamSynchronize(m->st));
-    double s = 0;
-    for (float v : l) s += v;
-    *loss_out = (float)(s / B);
-  }
-  return RH_OK;
+float mean_loss(const rh_mlp* m, int n) {
+  double s = 0;
+  for (int i = 0; i < n; ++i) s += m->h_out[i];
+  return (float)(s / n);
 }
 
 }  // namespace
@@ -520,79 +926,46 @@ int rh_mlp_create(int32_t batch_max, int32_t device, rh_mlp** out) {
   *out = nullptr;
   rh_mlp* m = new rh_mlp();
   m->bmax = batch_max;
-  const int wn[4] = {H, H, H, NOUT}, wk[4] = {KIN, H, H, H};
-  size_t nf = 0, nb = 0;
-  for (int l = 0; l < 4; ++l) {
-    m->wn[l] = wn[l];
-    m->wk[l] = wk[l];
-    nf += (size_t)7 * wn[l] * wk[l] + 5 * wn[l];  // w gw mw vw maskw + b gb mb vb
-    nb += (size_t)wn[l] * wk[l];
-  }
-  const size_t B = (size_t)batch_max;
-  nf += 4 * B * H + B * H * 2 + B * 3 * 2 + B * RH_MLP_IN + B;  // Z0-2, Z3(8), dA, dZf, y, target, xin, loss
-  nb += B * KIN + 3 * B * H + 3 * B * H + B * NOUT;              // X0, A0-2, dZb0-2, dZb3
-  int r = RH_OK;
+  m->device = device;
+  m->chunk = std::max(batch_max, kChunk);
+  const size_t B = (size_t)batch_max, chunk = (size_t)m->chunk;
+  const size_t parts = std::min<size_t>((B + 127) / 128, kMaxParts);
+  auto round256 = [](size_t b) { return (b + 255) / 256 * 256; };
+  int direct = 0;
+  if (cudaDeviceGetAttribute(&direct, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device) !=
+      cudaSuccess)
+    cudaGetLastError();
+  m->direct = direct != 0;
+  const size_t nx = direct ? 0 : round256(chunk * RH_MLP_IN * 4),
+               nt = direct ? 0 : round256(B * RH_MLP_OUT * 4),
+               no = round256(2 * chunk * RH_MLP_OUT * 4), ng = round256(kNPar * 4);
   if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreate(&m->st) != cudaSuccess ||
-      cudaMalloc(&m->P, nf * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&m->Pb, nb * sizeof(__nv_bfloat16)) != cudaSuccess ||
-      cudaMalloc(&m->gemm_err, sizeof(int)) != cudaSuccess ||
-      cudaMemset(m->gemm_err, 0, sizeof(int)) != cudaSuccess ||
-      cudaFuncSetAttribute(gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           tc::kSmemA + tc::kSmemB) != cudaSuccess) {
+      cudaMalloc(&m->P, (3 + parts) * (size_t)kNPar * sizeof(float)) != cudaSuccess ||
+      cudaMalloc(&m->img, kImgBytes) != cudaSuccess ||
+      cudaHostAlloc(&m->host, 2 * nx + nt + no + ng + 256, cudaHostAllocMapped) != cudaSuccess ||
+      cudaEventCreateWithFlags(&m->ev[0], cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&m->ev[1], cudaEventDisableTiming) != cudaSuccess ||
+      cudaFuncSetAttribute(mlp_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           RowsSmem::bytes(true)) != cudaSuccess ||
+      cudaFuncSetAttribute(mlp_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           RowsSmem::bytes(false)) != cudaSuccess ||
+      cudaMemset(m->P, 0, 3 * (size_t)kNPar * sizeof(float)) != cudaSuccess ||
+      cudaMemset(m->img, 0, kImgBytes) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
     m->err = "allocation failed";
-    r = RH_ERR_NOMEM;
-  }
-  if (r == RH_OK) {
-    cudaMemset(m->P, 0, nf * sizeof(float));
-    cudaMemset(m->Pb, 0, nb * sizeof(__nv_bfloat16));
-    float* p = m->P;
-    __nv_bfloat16* pb = m->Pb;
-    for (int l = 0; l < 4; ++l) {
-      const size_t nw = (size_t)wn[l] * wk[l];
-      m->w[l] = p; p += nw;
-      m->gw[l] = p; p += nw;
-      m->mw[l] = p; p += nw;
-      m->vw[l] = p; p += nw;
-      m->maskw[l] = p; p += nw;
-      m->b[l] = p; p += wn[l];
-      m->gb[l] = p; p += wn[l];
-      m->mb[l] = p; p += wn[l];
-      m->vb[l] = p; p += wn[l];
-      p += (size_t)2 * nw;  // spare (keeps the arithmetic above honest)
-      p += wn[l];
-      m->wb[l] = pb; pb += nw;
-    }
-    m->Z[0] = p; p += B * H;
-    m->Z[1] = p; p += B * H;
-    m->Z[2] = p; p += B * H;
-    m->Z[3] = p; p += B * H;  // only B*NOUT used
-    m->dA = p; p += B * H;
-    m->dZf = p; p += B * H;
-    m->y = p; p += B * 3;
-    m->target = p; p += B * 3;
-    m->xin = p; p += B * RH_MLP_IN;
-    m->loss = p; p += B;
-    m->X0 = pb; pb += B * KIN;
-    for (int l = 0; l < 3; ++l) { m->A[l] = pb; pb += B * H; }
-    for (int l = 0; l < 3; ++l) { m->dZb[l] = pb; pb += B * H; }
-    m->dZb[3] = pb; pb += B * NOUT;
-    // masks: real weights 1, padding 0 (layer 1 inputs >= 4, layer 4 outputs >= 3)
-    for (int l = 0; l < 4; ++l) {
-      std::vector<float> mk((size_t)wn[l] * wk[l], 1.f);
-      for (int n = 0; n < wn[l]; ++n)
-        for (int k = 0; k < wk[l]; ++k)
-          if ((l == 0 && k >= RH_MLP_IN) || (l == 3 && n >= RH_MLP_OUT)) mk[(size_t)n * wk[l] + k] = 0.f;
-      cudaMemcpy(m->maskw[l], mk.data(), mk.size() * sizeof(float), cudaMemcpyHostToDevice);
-    }
-    if (cudaDeviceSynchronize() != cudaSuccess) {
-      m->err = "initialisation failed";
-      r = RH_ERR_CUDA;
-    }
-  }
-  if (r != RH_OK) {
+    cudaGetLastError();
     rh_mlp_destroy(m);
-    return r;
+    return RH_ERR_NOMEM;
   }
+  m->w = m->P;
+  m->m = m->w + kNPar;
+  m->v = m->m + kNPar;
+  m->part = m->v + kNPar;
+  m->h_x = reinterpret_cast<float*>(m->host);  // two chunks
+  m->h_t = reinterpret_cast<float*>(m->host + 2 * nx);
+  m->h_out = reinterpret_cast<float*>(m->host + 2 * nx + nt);
+  m->h_g = reinterpret_cast<float*>(m->host + 2 * nx + nt + no);
+  m->h_err = reinterpret_cast<int*>(m->host + 2 * nx + nt + no + ng);
+  *m->h_err = 0;
   *out = m;
   return RH_OK;
 }
@@ -601,8 +974,10 @@ int rh_mlp_destroy(rh_mlp* m) {
   if (!m) return RH_ERR_ARG;
   if (m->st) cudaStreamSynchronize(m->st);
   cudaFree(m->P);
-  cudaFree(m->Pb);
-  cudaFree(m->gemm_err);
+  cudaFree(m->img);
+  if (m->host) cudaFreeHost(m->host);
+  for (cudaEvent_t e : m->ev)
+    if (e) cudaEventDestroy(e);
   if (m->st) cudaStreamDestroy(m->st);
   delete m;
   return RH_OK;
@@ -610,30 +985,17 @@ int rh_mlp_destroy(rh_mlp* m) {
 
 int rh_mlp_param_count(const rh_mlp* m, int32_t* n) {
   if (!m || !n) return RH_ERR_ARG;
-  int s = 0;
-  for (int l = 0; l < 4; ++l) s += m->wn[l] * m->wk[l] + m->wn[l];
-  *n = s;
+  *n = kNPar;
   return RH_OK;
 }
 
 // Parameter order: for each layer, W (n x k row-major, padded) then b (n).
 int rh_mlp_set_params(rh_mlp* m, const float* params) {
   if (!m || !params) return RH_ERR_ARG;
-  const float* p = params;
-  for (int l = 0; l < 4; ++l) {
-    const size_t nw = (size_t)m->wn[l] * m->wk[l];
-    MCK(cudaMemcpy(m->w[l], p, nw * sizeof(float), cudaMemcpyHostToDevice));
-    p += nw;
-    MCK(cudaMemcpy(m->b[l], p, m->wn[l] * sizeof(float), cudaMemcpyHostToDevice));
-    p += m->wn[l];
-    // apply the padding mask and refresh BF16 copies; reset Adam
-    adam_update<<<blocks(nw, 256), 256, 0, m->st>>>(m->w[l], m->gw[l], m->mw[l], m->vw[l], m->wb[l],
-                                                   m->maskw[l], (int)nw, 0.f, 0.f, 0.f, 1.f, 1.f, 1.f);
-    MCK(cudaMemsetAsync(m->mw[l], 0, nw * sizeof(float), m->st));
-    MCK(cudaMemsetAsync(m->vw[l], 0, nw * sizeof(float), m->st));
-    MCK(cudaMemsetAsync(m->mb[l], 0, m->wn[l] * sizeof(float), m->st));
-    MCK(cudaMemsetAsync(m->vb[l], 0, m->wn[l] * sizeof(float), m->st));
-  }
+  MCK(cudaMemcpyAsync(m->w, params, kNPar * sizeof(float), cudaMemcpyHostToDevice, m->st));
+  mlp_load<<<blocks(kNPar, 256), 256, 0, m->st>>>(m->w, m->img);
+  MCK(cudaGetLastError());
+  MCK(cudaMemsetAsync(m->m, 0, 2 * (size_t)kNPar * sizeof(float), m->st));  // Adam's moments
   m->step = 0;
   MCK(cudaStreamSynchronize(m->st));
   return RH_OK;
@@ -641,70 +1003,88 @@ int rh_mlp_set_params(rh_mlp* m, const float* params) {
 
 int rh_mlp_get_params(rh_mlp* m, float* params) {
   if (!m || !params) return RH_ERR_ARG;
+  MCK(cudaMemcpyAsync(params, m->w, kNPar * sizeof(float), cudaMemcpyDeviceToHost, m->st));
   MCK(cudaStreamSynchronize(m->st));
-  float* p = params;
-  for (int l = 0; l < 4; ++l) {
-    const size_t nw = (size_t)m->wn[l] * m->wk[l];
-    MCK(cudaMemcpy(p, m->w[l], nw * sizeof(float), cudaMemcpyDeviceToHost));
-    p += nw;
-    MCK(cudaMemcpy(p, m->b[l], m->wn[l] * sizeof(float), cudaMemcpyDeviceToHost));
-    p += m->wn[l];
-  }
   return RH_OK;
 }
 
+// The sweep runs in launches of `chunk` samples that write their outputs to
+// two mapped host buffers in turn, so that the host copies one chunk's
+// outputs out while the next one runs.
 int rh_mlp_forward(rh_mlp* m, const float* x, int32_t n, float* y) {
   if (!m || !x || !y || n <= 0) return RH_ERR_ARG;
-  for (int32_t off = 0; off < n; off += m->bmax) {
-    const int B = (int)std::min<int64_t>(m->bmax, n - off);
-    int r = run_loss(m, B, x + (size_t)off * RH_MLP_IN, nullptr, nullptr);
-    if (r) return r;
-    MCK(cudaMemcpyAsync(y + (size_t)off * 3, m->y, sizeof(float) * 3 * B, cudaMemcpyDeviceToHost,
-                        m->st));
+  const int64_t C = m->chunk;
+  const int nch = (int)((n + C - 1) / C);
+  auto rows = [&](int c) { return (int)std::min<int64_t>(C, n - c * C); };
+  auto buffer = [&](int c) { return m->h_out + (size_t)(c & 1) * C * RH_MLP_OUT; };
+  auto launch = [&](int c) -> int {
+    RowsArgs a{};
+    a.img = m->img;
+    a.params = m->w;
+    a.x = reachable(m, x + (size_t)c * C * RH_MLP_IN, (size_t)rows(c) * RH_MLP_IN,
+                    m->h_x + (size_t)(c & 1) * C * RH_MLP_IN);
+    a.y = buffer(c);
+    a.n = rows(c);
+    a.err = m->h_err;
+    const int tiles = (a.n + 127) / 128;
+    mlp_rows<false><<<std::min(tiles, kMaxParts), kRowThreads, RowsSmem::bytes(false), m->st>>>(a);
+    MCK(cudaGetLastError());
+    MCK(cudaEventRecord(m->ev[c & 1], m->st));
+    return RH_OK;
+  };
+  int r = launch(0);
+  for (int c = 0; c < nch && r == RH_OK; ++c) {
+    // the next chunk's buffers: last used by chunk c - 1, already copied out
+    if (c + 1 < nch) r = launch(c + 1);
+    if (r == RH_OK) r = ck(m, cudaEventSynchronize(m->ev[c & 1]), "forward");
+    if (r == RH_OK)
+      memcpy(y + (size_t)c * C * RH_MLP_OUT, buffer(c), sizeof(float) * RH_MLP_OUT * rows(c));
   }
-  MCK(cudaStreamSynchronize(m->st));
-  return check_gemm(m);
+  if (r != RH_OK) {
+    cudaStreamSynchronize(m->st);  // no launch still reads or writes host memory
+    return r;
+  }
+  return check_wait(m);
 }
 
 int rh_mlp_gradients(rh_mlp* m, const float* x, const float* target, int32_t n, float* grads,
                      float* loss) {
   if (!m || !x || !target || n <= 0 || n > m->bmax) return RH_ERR_ARG;
-  int r = run_loss(m, n, x, target, loss);
+  int parts = 0;
+  int r = train_pass(m, x, target, n, &parts);
   if (r) return r;
-  if ((r = backward(m, n))) return r;
   if (grads) {
-    MCK(cudaStreamSynchronize(m->st));
-    if ((r = check_gemm(m))) return r;
-    float* p = grads;
-    for (int l = 0; l < 4; ++l) {
-      const size_t nw = (size_t)m->wn[l] * m->wk[l];
-      MCK(cudaMemcpy(p, m->gw[l], nw * sizeof(float), cudaMemcpyDeviceToHost));
-      p += nw;
-      MCK(cudaMemcpy(p, m->gb[l], m->wn[l] * sizeof(float), cudaMemcpyDeviceToHost));
-      p += m->wn[l];
-    }
+    mlp_finish<<<blocks(kNPar, 256), 256, 0, m->st>>>(m->part, parts, m->h_g, nullptr, nullptr,
+                                                      nullptr, nullptr, AdamStep{});
+    r = ck(m, cudaGetLastError(), "gradients");
   }
+  const int rs = ck(m, cudaStreamSynchronize(m->st), "gradients");
+  if (r) return r;
+  if (rs) return rs;
+  if ((r = check_wait(m))) return r;
+  if (grads) memcpy(grads, m->h_g, kNPar * sizeof(float));
+  if (loss) *loss = mean_loss(m, n);
   return RH_OK;
 }
 
 int rh_mlp_train_step(rh_mlp* m, const float* x, const float* target, int32_t n, float lr,
                       float* loss) {
-  int r = rh_mlp_gradients(m, x, target, n, nullptr, loss);
+  if (!m || !x || !target || n <= 0 || n > m->bmax) return RH_ERR_ARG;
+  int parts = 0;
+  int r = train_pass(m, x, target, n, &parts);
   if (r) return r;
   m->step += 1;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  const float bc1 = 1.f - powf(b1, (float)m->step), bc2 = 1.f - powf(b2, (float)m->step);
-  for (int l = 0; l < 4; ++l) {
-    const int nw = m->wn[l] * m->wk[l];
-    adam_update<<<blocks(nw, 256), 256, 0, m->st>>>(m->w[l], m->gw[l], m->mw[l], m->vw[l], m->wb[l],
-                                                   m->maskw[l], nw, lr, b1, b2, eps, bc1, bc2);
-    adam_update<<<blocks(m->wn[l], 128), 128, 0, m->st>>>(m->b[l], m->gb[l], m->mb[l], m->vb[l],
-                                                         nullptr, nullptr, m->wn[l], lr, b1, b2, eps,
-                                                         bc1, bc2);
-  }
-  MCK(cudaGetLastError());
-  MCK(cudaStreamSynchronize(m->st));
-  return check_gemm(m);
+  const AdamStep s{lr, b1, b2, eps, 1.f - powf(b1, (float)m->step), 1.f - powf(b2, (float)m->step)};
+  mlp_finish<<<blocks(kNPar, 256), 256, 0, m->st>>>(m->part, parts, nullptr, m->w, m->m, m->v,
+                                                    m->img, s);
+  r = ck(m, cudaGetLastError(), "training step");
+  const int rs = ck(m, cudaStreamSynchronize(m->st), "training step");
+  if (r) return r;
+  if (rs) return rs;
+  if ((r = check_wait(m))) return r;
+  if (loss) *loss = mean_loss(m, n);
+  return RH_OK;
 }
 
 int rh_mlp_last_error(const rh_mlp* m, char* buf, size_t n) {
@@ -723,71 +1103,12 @@ int rh_mlp_last_error(const rh_mlp* m, char* buf, size_t n) {
 // loop that budgets device memory up front, or a caller that must not pay the
 // device-wide synchronisation an allocation can imply.  rh_mlp_forward_noalloc
 // serves them: the caller brings the parameters, inputs and outputs in device
-// memory, and the intermediate values (BF16 weight copies, packed inputs,
-// pre-activations, activations, output-layer terms) live in the fixed array
-// below, which is part of the library image on every device that loads it.
-
-static __device__ __align__(256) unsigned char g_forward_scratch[RH_MLP_NOALLOC_SCRATCH_BYTES];
+// memory, and one launch of mlp_rows converts the weights into shared memory
+// and keeps every intermediate value there.
 
 namespace {
 
-// Byte offsets inside the scratch array, each a multiple of 256.
-constexpr size_t kNaRows = RH_MLP_NOALLOC_MAX_BATCH;
-constexpr size_t kNaWeights = (size_t)H * KIN + 2 * (size_t)H * H + (size_t)NOUT * H;
-constexpr size_t round256(size_t b) { return (b + 255) / 256 * 256; }
-constexpr size_t kOffW = 0;
-constexpr size_t kOffX0 = kOffW + round256(kNaWeights * 2);
-constexpr size_t kOffZ = kOffX0 + round256(kNaRows * KIN * 2);
-constexpr size_t kOffA = kOffZ + round256(kNaRows * H * 4);
-constexpr size_t kOffDz = kOffA + round256(kNaRows * H * 2);
-constexpr size_t kOffDzb = kOffDz + round256(kNaRows * NOUT * 4);
-constexpr size_t kNaEnd = kOffDzb + round256(kNaRows * NOUT * 2);
-static_assert(kNaEnd <= RH_MLP_NOALLOC_SCRATCH_BYTES, "scratch layout exceeds the array");
-
-// FP32 weights of one layer -> BF16, padding entries (layer 1 inputs >= 4,
-// layer 4 outputs >= 3) forced to zero, as rh_mlp_set_params does.
-__global__ void weights_to_bf16(const float* w, __nv_bfloat16* wb, int n, int k, int nvalid,
-                                int kvalid) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n * k) return;
-  const int r = i / k, c = i % k;
-  wb[i] = __float2bfloat16(r < nvalid && c < kvalid ? w[i] : 0.f);
-}
-
 constexpr int kMaxDevices = 64;
-// The device address of the scratch array belongs to one CUDA context.  The
-// cache holds it per device together with the id of the context that was
-// current when it was looked up; a call from another context on that device
-// (a context the caller made current, or the primary context created anew
-// after cudaDeviceReset) looks it up again.
-std::mutex g_scratch_mu;
-void* g_scratch_addr[kMaxDevices] = {};
-unsigned long long g_scratch_ctx[kMaxDevices] = {};
-
-// Id of the calling thread's current context (cuCtxGetCurrent + cuCtxGetId,
-// reached through the runtime's driver entry points so that the library does
-// not link the driver library itself); false where it cannot be had.
-bool current_context_id(unsigned long long* id) {
-  using GetCurrentFn = CUresult (*)(CUcontext*);
-  using GetIdFn = CUresult (*)(CUcontext, unsigned long long*);
-  static GetCurrentFn get_current = nullptr;
-  static GetIdFn get_id = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) ==
-            cudaSuccess && q == cudaDriverEntryPointSuccess)
-      get_current = reinterpret_cast<GetCurrentFn>(f);
-    f = nullptr;
-    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) ==
-            cudaSuccess && q == cudaDriverEntryPointSuccess)
-      get_id = reinterpret_cast<GetIdFn>(f);
-  });
-  CUcontext ctx = nullptr;
-  if (!get_current || !get_id || get_current(&ctx) != CUDA_SUCCESS || !ctx) return false;
-  return get_id(ctx, id) == CUDA_SUCCESS;
-}
 
 void na_msg(char* err, size_t len, const char* fmt, ...) __attribute__((format(printf, 3, 4)));
 void na_msg(char* err, size_t len, const char* fmt, ...) {
@@ -818,9 +1139,8 @@ extern "C" int rh_mlp_forward_noalloc(const float* d_params, const float* d_x, i
   }
   if (n <= 0 || n > RH_MLP_NOALLOC_MAX_BATCH) {
     na_msg(err, err_len,
-           "rh_mlp_forward_noalloc: n = %d is outside 1..%d, the largest batch its fixed "
-           "%d-byte scratch array holds; split the batch",
-           (int)n, RH_MLP_NOALLOC_MAX_BATCH, RH_MLP_NOALLOC_SCRATCH_BYTES);
+           "rh_mlp_forward_noalloc: n = %d is outside 1..%d; split the batch", (int)n,
+           RH_MLP_NOALLOC_MAX_BATCH);
     return RH_ERR_ARG;
   }
   int dev = -1;
@@ -837,75 +1157,20 @@ extern "C" int rh_mlp_forward_noalloc(const float* d_params, const float* d_x, i
            dev);
     return RH_ERR_ARG;
   }
-  // Set-up, once per device (and context), with that device current: the
-  // scratch array's device address.  Later calls from the same context reuse
-  // the cached address.
-  void* base = nullptr;
-  {
-    // the pointer checks above ran runtime calls on this thread, so its
-    // context is current; without a context id the address is looked up
-    // on every call
-    unsigned long long ctx = 0;
-    const bool known_ctx = current_context_id(&ctx);
-    std::lock_guard<std::mutex> lock(g_scratch_mu);
-    if (!g_scratch_addr[dev] || !known_ctx || g_scratch_ctx[dev] != ctx) {
-      void* p = nullptr;
-      e = cudaGetSymbolAddress(&p, g_forward_scratch);
-      if (e != cudaSuccess || !p) {
-        na_msg(err, err_len, "rh_mlp_forward_noalloc: cudaGetSymbolAddress failed on device %d: %s",
-               dev, cudaGetErrorString(e));
-        return RH_ERR_CUDA;
-      }
-      g_scratch_addr[dev] = p;
-      g_scratch_ctx[dev] = known_ctx ? ctx : 0;
-    }
-    base = g_scratch_addr[dev];
-  }
-  unsigned char* s = static_cast<unsigned char*>(base);
-  __nv_bfloat16* wb = reinterpret_cast<__nv_bfloat16*>(s + kOffW);
-  __nv_bfloat16* X0 = reinterpret_cast<__nv_bfloat16*>(s + kOffX0);
-  float* Z = reinterpret_cast<float*>(s + kOffZ);
-  __nv_bfloat16* A = reinterpret_cast<__nv_bfloat16*>(s + kOffA);
-  float* dz = reinterpret_cast<float*>(s + kOffDz);
-  __nv_bfloat16* dzb = reinterpret_cast<__nv_bfloat16*>(s + kOffDzb);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-
-  // Every scratch element read below is written earlier in this call, so the
-  // previous call's contents never leak into the result and nothing needs
-  // clearing.
-  const int wn[4] = {H, H, H, NOUT}, wk[4] = {KIN, H, H, H};
-  const float* wl[4];
-  const float* bl[4];
-  __nv_bfloat16* wbl[4];
-  {
-    const float* p = d_params;
-    __nv_bfloat16* q = wb;
-    for (int l = 0; l < 4; ++l) {
-      const int nw = wn[l] * wk[l];
-      wl[l] = p;
-      bl[l] = p + nw;
-      wbl[l] = q;
-      p += nw + wn[l];
-      q += nw;
-      weights_to_bf16<<<blocks(nw, 256), 256, 0, st>>>(wl[l], wbl[l], wn[l], wk[l],
-                                                        l == 3 ? RH_MLP_OUT : wn[l],
-                                                        l == 0 ? RH_MLP_IN : wk[l]);
-    }
+  e = cudaFuncSetAttribute(mlp_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           RowsSmem::bytes(false));
+  if (e != cudaSuccess) {
+    na_msg(err, err_len, "rh_mlp_forward_noalloc: set-up failed on device %d: %s", dev,
+           cudaGetErrorString(e));
+    return RH_ERR_CUDA;
   }
-  const int B = n;
-  pack_inputs<<<blocks((int64_t)B * KIN, 256), 256, 0, st>>>(d_x, X0, B);
-  const __nv_bfloat16* in = X0;
-  for (int l = 0; l < 4; ++l) {
-    const int kin = wk[l], nout = wn[l];
-    const int tiles = ((B + 15) / 16) * ((nout + 7) / 8);
-    gemm_bf16<<<blocks((int64_t)tiles * 32, 128), 128, 0, st>>>(in, kin, 1, wbl[l], 1, kin, Z, nout,
-                                                                B, nout, kin, 0);
-    if (l < 3) {
-      bias_relu<<<blocks((int64_t)B * H, 256), 256, 0, st>>>(Z, bl[l], A, B, H);
-      in = A;
-    }
-  }
-  output_loss<<<blocks(B, 128), 128, 0, st>>>(Z, bl[3], nullptr, d_y, dz, dzb, nullptr, B);
+  RowsArgs a{};
+  a.params = d_params;
+  a.x = d_x;
+  a.y = d_y;
+  a.n = n;
+  mlp_rows<false><<<(n + 127) / 128, kRowThreads, RowsSmem::bytes(false), st>>>(a);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     na_msg(err, err_len, "rh_mlp_forward_noalloc: launch failed: %s", cudaGetErrorString(e));
