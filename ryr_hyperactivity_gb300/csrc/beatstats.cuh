@@ -67,12 +67,11 @@ __host__ __device__ inline void beat_finish(const BeatTracker& b, rh_beat_stats*
   out->pad = 0;
 }
 
-// One per-step sample.  Returns 1 when a beat completed; its statistics are
-// written to *out.
-__host__ __device__ inline int beat_on_step(BeatTracker& b, double t, double v, double pcl,
-                                            rh_beat_stats* out) {
+// One per-step sample of beat k (-1 before the first stimulus).  Returns 1
+// when a beat completed; its statistics are written to *out.
+__host__ __device__ inline int beat_sample(BeatTracker& b, int k, double t, double v,
+                                           rh_beat_stats* out) {
   int done = 0;
-  int k = t < kStimStart ? -1 : (int)floor((t - kStimStart) / pcl);
   if (k != b.beat && k >= 0) {
     if (b.beat >= 0) {
       beat_finish(b, out);
@@ -118,6 +117,10 @@ __host__ __device__ inline int beat_on_step(BeatTracker& b, double t, double v, 
     }
   }
   return done;
+}
+__host__ __device__ inline int beat_on_step(BeatTracker& b, double t, double v, double pcl,
+                                            rh_beat_stats* out) {
+  return beat_sample(b, t < kStimStart ? -1 : (int)floor((t - kStimStart) / pcl), t, v, out);
 }
 
 // One output record (the 45 wholecell columns).

@@ -244,76 +244,99 @@ __host__ __device__ inline bool step_coef(StepCoef<double>& k, const rh_membrane
   return t < c.tend;
 }
 
-// Output-step reductions -> the 45 wholecell columns (:931-1072).
-__host__ __device__ inline void wholecell_columns(double* w, const double* o, const rh_membrane& m,
-                                                  int nin, double dt) {
+// Output-step reductions o[NOUT] -> the 45 wholecell columns (:931-1072), by
+// one full warp: lane q holds statistic q and divides it (one SIMT quotient
+// where 40 in one lane took the record's lane 11 us), lane 0 writes.
+__device__ inline void wholecell_columns_warp(double* w, const double* o, const rh_membrane& m,
+                                              int nin, double dt, int lane) {
+  auto at = [&](double x, int idx) { return __shfl_sync(0xffffffffu, x, idx - P_STEP_END); };
   const double N = nin;
-  double cit = o[O_CI - P_STEP_END] / 8. / N;
-  double cproxit = o[O_CP - P_STEP_END] / N;
-  double cjsrt = o[O_CJSR - P_STEP_END] / N;
-  double csqnbt = o[O_CJSRB - P_STEP_END] / N;
-  double cnsrt = o[O_CNSR - P_STEP_END] / 8. / N;
-  double poto = o[O_PO - P_STEP_END] / N;
-  double pbcto = o[O_NCB - P_STEP_END] / N / 100.;
-  double catft = o[O_CATF - P_STEP_END] / 8. / N;
-  double catst = o[O_CATS - P_STEP_END] / 8. / N;
-  double casrt = o[O_CASR - P_STEP_END] / 8. / N;
-  double camyot = o[O_CAMYO - P_STEP_END] / 8. / N;
-  double cacalt = o[O_CACAL - P_STEP_END] / 8. / N;
-  double leakt = o[O_LEAK - P_STEP_END] / 8. / N;
-  double upt = o[O_UP - P_STEP_END] / 8. / N;
-  double ire = o[O_XIRE - P_STEP_END] / N;
-  double ncxfwd = o[O_NCXFWD - P_STEP_END] / N;
-  double outancx = o[O_ANCX - P_STEP_END] / N;
-  double casart = o[O_CASAR - P_STEP_END] / N;
-  double casarht = o[O_CASARH - P_STEP_END] / N;
-  double casarjt = o[O_CASARJ - P_STEP_END] / N;
-  double casarhjt = o[O_CASARHJ - P_STEP_END] / N;
+  const int idx = P_STEP_END + lane;
+  // per-sub-voxel sums: over the 8 sub-voxels too (x / 8 is exact)
+  const bool sub = idx == O_CNSR || idx == O_CI || (idx >= O_CATF && idx <= O_UP);
+  const double x = o[lane];
+  // the lane of O_NOU, which is not divided, takes the window's steps
+  const double q = Math<double>::div(idx == O_NOU ? OUTT : sub ? x * 0.125 : x,
+                                     idx == O_NOU ? dt : N);
+  const double steps = at(q, O_NOU);
+  const double q2 = Math<double>::div(idx == O_NCB   ? q
+                                      : idx == O_NOU ? m.out_ncx
+                                      : idx == O_NOB ? m.out_ica
+                                      : idx == O_NCU ? m.out_ina
+                                                     : 1.0,
+                                      idx == O_NCB ? 100. : steps);
+  const double cit = at(q, O_CI), cproxit = at(q, O_CP), cjsrt = at(q, O_CJSR);
+  const double csqnbt = at(q, O_CJSRB), cnsrt = at(q, O_CNSR), poto = at(q, O_PO);
+  const double pbcto = at(q2, O_NCB), catft = at(q, O_CATF), catst = at(q, O_CATS);
+  const double casrt = at(q, O_CASR), camyot = at(q, O_CAMYO), cacalt = at(q, O_CACAL);
+  const double leakt = at(q, O_LEAK), upt = at(q, O_UP), ire = at(q, O_XIRE);
+  const double ncxfwd = at(q, O_NCXFWD), outancx = at(q, O_ANCX), casart = at(q, O_CASAR);
+  const double casarht = at(q, O_CASARH), casarjt = at(q, O_CASARJ), casarhjt = at(q, O_CASARHJ);
+  const double ncx = at(q2, O_NOU), ica = at(q2, O_NOB), ina = at(q2, O_NCU);
   const double csubt = m.csubt;
-  double total_ca = (cit + catft + catst + casrt + camyot + cacalt) * VI * 8. +
-                    (csubt + casart + casarht) * VS + (cproxit + casarjt + casarhjt) * VP +
-                    (cnsrt)*VNSR * 8. + (cjsrt + csqnbt) * VJSR;
-  double total_ci = (cit + catft + catst + casrt + camyot + cacalt) * VI * 8. +
-                    (csubt + casart + casarht) * VS + (cproxit + casarjt + casarhjt) * VP;
-  w[0] = m.t;
-  w[1] = cit;
-  w[2] = m.v;
-  w[3] = m.out_ncx / (OUTT / dt);
-  w[4] = m.out_ica / (OUTT / dt);
-  w[5] = cproxit;
-  w[6] = csubt;
-  w[7] = cjsrt;
-  w[8] = cnsrt;
-  w[9] = poto;
-  w[10] = m.xnai;
-  w[11] = m.xiks;
-  w[12] = m.xikr;
-  w[13] = m.xik1;
-  w[14] = m.xinak;
-  w[15] = m.xitos;
-  w[16] = m.xitof;
-  w[17] = m.out_ina / (OUTT / dt);
-  w[18] = m.xr;
-  w[19] = ncxfwd * (VS / VP);
-  w[20] = pbcto;
-  w[21] = cacalt;
-  w[22] = catft;
-  w[23] = leakt;
-  w[24] = upt;
-  w[25] = ire;
-  w[26] = o[O_NOU - P_STEP_END];
-  w[27] = o[O_NOB - P_STEP_END];
-  w[28] = o[O_NCU - P_STEP_END];
-  w[29] = o[O_NCB - P_STEP_END];
-  for (int q = 0; q < 7; ++q) w[30 + q] = o[O_TN1 - P_STEP_END + q];
-  w[37] = outancx;
-  w[38] = m.xs1;
-  w[39] = m.qks;
-  w[40] = (double)m.sparksum;
-  w[41] = catst;
-  w[42] = csqnbt;
-  w[43] = total_ci;
-  w[44] = total_ca;
+  const double total_ci = (cit + catft + catst + casrt + camyot + cacalt) * VI * 8. +
+                          (csubt + casart + casarht) * VS + (cproxit + casarjt + casarhjt) * VP;
+  const double total_ca = total_ci + (cnsrt)*VNSR * 8. + (cjsrt + csqnbt) * VJSR;
+  if (lane == 0) {
+    w[0] = m.t;
+    w[1] = cit;
+    w[2] = m.v;
+    w[3] = ncx;
+    w[4] = ica;
+    w[5] = cproxit;
+    w[6] = csubt;
+    w[7] = cjsrt;
+    w[8] = cnsrt;
+    w[9] = poto;
+    w[10] = m.xnai;
+    w[11] = m.xiks;
+    w[12] = m.xikr;
+    w[13] = m.xik1;
+    w[14] = m.xinak;
+    w[15] = m.xitos;
+    w[16] = m.xitof;
+    w[17] = ina;
+    w[18] = m.xr;
+    w[19] = ncxfwd * (VS / VP);
+    w[20] = pbcto;
+    w[21] = cacalt;
+    w[22] = catft;
+    w[23] = leakt;
+    w[24] = upt;
+    w[25] = ire;
+    w[26] = o[O_NOU - P_STEP_END];
+    w[27] = o[O_NOB - P_STEP_END];
+    w[28] = o[O_NCU - P_STEP_END];
+    w[29] = o[O_NCB - P_STEP_END];
+    for (int k = 0; k < 7; ++k) w[30 + k] = o[O_TN1 - P_STEP_END + k];
+    w[37] = outancx;
+    w[38] = m.xs1;
+    w[39] = m.qks;
+    w[40] = (double)m.sparksum;
+    w[41] = catst;
+    w[42] = csqnbt;
+    w[43] = total_ci;
+    w[44] = total_ca;
+  }
+}
+
+// Output-step partials of one cell, one row per warp of each of its tiles:
+// lane q sums statistic q over the rows in order into o[q]; the ci > 1000
+// flag (the last one) is a maximum.  A warp's FP64 additions cost the same
+// with one lane or 32, so a statistic per lane beats a row per lane with a
+// reduction for each of 33 statistics (441 rows: 441 against 630).
+__device__ inline void output_sums_warp(const double* partials, int nrows, double* o, int lane) {
+  static_assert(O_CIHIGH - P_STEP_END == NOUT - 1 && NOUT - 1 == 32, "one statistic per lane");
+  double s = 0.0;
+  bool high = false;
+#pragma unroll 4
+  for (int r = 0; r < nrows; ++r) s += __ldcg(partials + (size_t)r * P_COUNT + P_STEP_END + lane);
+  for (int r = lane; r < nrows; r += 32)
+    high |= __ldcg(partials + (size_t)r * P_COUNT + O_CIHIGH) > 0.0;
+  high = __any_sync(0xffffffffu, high);
+  o[lane] = s;
+  if (lane == 0) o[NOUT - 1] = high ? 1.0 : 0.0;
+  __syncwarp();
 }
 
 }  // namespace rh

@@ -41,6 +41,14 @@ struct ExpArg {
 
 enum { kSrcV = 0, kSrcVek = 1, kSrcNao = 2 };
 
+// a b + c d with its rounding fixed (the compiler may fuse either product).
+// Here and where __dmul_rn and __dadd_rn stand below, a product that is added
+// elsewhere is rounded first, so that the one-warp and the four-warp update
+// (cellwide.cuh) give the same bits.
+__device__ __forceinline__ double sum_of_products(double a, double b, double c, double d) {
+  return fma(a, b, __dmul_rn(c, d));
+}
+
 #define RH_MUL(c_, a_) {a_, c_, 1.0, 1.0, kSrcV, 0, 0, 0}
 #define RH_DIV(a_, d_) {a_, 1.0, d_, 1.0, kSrcV, 1, 0, 0}
 #define RH_NONE {0.0, 0.0, 1.0, 1.0, kSrcV, 0, 0, 0}
@@ -193,9 +201,9 @@ __device__ inline void membrane_pre_warp(rh_membrane& m, double dt, const CellCo
   P.rdt95 = w.get(6);
   // logarithms (lanes 0-2)
   const double lgv = log(w.r[lane]);
-  const double ena = (1.0 / FRT) * __shfl_sync(0xffffffffu, lgv, 0);
-  const double ek = (1.00 / FRT) * __shfl_sync(0xffffffffu, lgv, 1);
-  const double eks = (1.00 / FRT) * __shfl_sync(0xffffffffu, lgv, 2);
+  const double ena = __dmul_rn(1.0 / FRT, __shfl_sync(0xffffffffu, lgv, 0));
+  const double ek = __dmul_rn(1.00 / FRT, __shfl_sync(0xffffffffu, lgv, 1));
+  const double eks = __dmul_rn(1.00 / FRT, __shfl_sync(0xffffffffu, lgv, 2));
   const double pow_nak = w.get(3);  // pow(12/xnai, 1) = 12/xnai
   // fmods: stimulus phase (:689, iso :683) and the next update's window,
   // output, cadist and iso LCC flags (:1244, :777, :1002, :1213)
@@ -232,7 +240,7 @@ __device__ inline void membrane_pre_warp(rh_membrane& m, double dt, const CellCo
   const bool low = v < -40.0;
 
   // ---- round 2: first-level divisions ----
-  const double bm = 0.08 * E[1];
+  const double bm = __dmul_rn(0.08, E[1]);
   double ah, bh, aj, bj, am;
   w.open(20);
   w.put(0, 0.32 * (v + 47.13), 1.0 - E[0]);                    // am
@@ -264,9 +272,9 @@ __device__ inline void membrane_pre_warp(rh_membrane& m, double dt, const CellCo
   P.rdth95 = w.get(19);
   am = w.get(0);
   if (low) {
-    ah = 0.135 * E[2];
-    bh = 3.56 * E[3] + 310000.0 * E[4];
-    aj = (-127140.0 * E[5] - 0.00003474 * E[6]) * w.get(1);
+    ah = __dmul_rn(0.135, E[2]);
+    bh = sum_of_products(3.56, E[3], 310000.0, E[4]);
+    aj = __dmul_rn(sum_of_products(-127140.0, E[5], -0.00003474, E[6]), w.get(1));
     bj = w.get(2);
   } else {
     ah = 0.00;
@@ -328,7 +336,7 @@ __device__ inline void membrane_pre_warp(rh_membrane& m, double dt, const CellCo
   //      every lane) ----
   const double gna = 15;
   const double gnaleak = 0.3e-3 * 5;
-  P.xina = gna * m.xh * m.xj * m.xm * m.xm * m.xm * (v - ena) + gnaleak * (v - ena);
+  P.xina = sum_of_products(gna * m.xh * m.xj * m.xm * m.xm * m.xm, v - ena, gnaleak, v - ena);
   m.xh = rh_ - (rh_ - m.xh) * G[0];
   m.xj = rj_ - (rj_ - m.xj) * G[1];
   m.xm = rm_ - (rm_ - m.xm) * G[2];
@@ -376,13 +384,17 @@ __device__ inline void membrane_post_warp(rh_membrane& m, double dt, const CellC
   const double xrr = 1.0 * (1.0 / wcainv / conv) / 1000.0;
   const double dnai = -xrr * (P.xina + 3.0 * P.xinak + 3.0 * m.xinacato);
   m.xnai = xnai + dnai * dt;
-  const double dvh = -(P.xina + P.xik1 + 1 * P.xikr + 1 * P.xiks + P.xitos + 1 * P.xitof +
-                       1. * m.xinacato + 1 * m.xicatto + P.xinak) +
-                     P.stim;
+  // sums of currents that are products themselves: each rounded before it is
+  // added, whatever the compiler could fuse
+  double s6 = __dadd_rn(P.xina, P.xik1);
+  s6 = __dadd_rn(__dadd_rn(s6, P.xikr), P.xiks);
+  s6 = __dadd_rn(__dadd_rn(s6, P.xitos), P.xitof);
+  const double sum = __dadd_rn(__dadd_rn(s6, m.xinacato), m.xicatto);
+  const double dvh = -__dadd_rn(sum, P.xinak) + P.stim;
   m.v = protocol_voltage(c, t, dt, v + dvh * dt);
-  m.out_ica += m.xicatto;
-  m.out_ncx += m.xinacato;
-  m.out_ina += P.xina;
+  m.out_ica = __dadd_rn(m.out_ica, m.xicatto);
+  m.out_ncx = __dadd_rn(m.out_ncx, m.xinacato);
+  m.out_ina = __dadd_rn(m.out_ina, P.xina);
   m.xina = P.xina;
   m.xiks = P.xiks;
   m.xikr = P.xikr;
@@ -514,19 +526,13 @@ __device__ inline bool step_coef_warp(StepCoef<double>& k, const rh_membrane& m,
 // K = 0.28^3, qks_inf = 0.2 (c3 + K + num c3) / (c3 + K), so
 //   dqks = dt (0.2 (c3 + K + num c3) - qks (c3 + K)) / ((c3 + K) tauqks),
 // the reference's three quotients (q28, qks_inf, the increment) folded into
-// one (equal in exact arithmetic; the last bits differ).  `s` as in
-// membrane_post_warp; all lanes return the increment.
-__device__ inline double qks_increment_warp(double csubt, double qks, double num, double tauqks,
-                                            double dt, double* s) {
-  const int lane = threadIdx.x & 31;
-  WarpSlots w{s, s + 32, s + 64, lane};
+// one (equal in exact arithmetic; the last bits differ).
+__device__ inline double qks_increment(double csubt, double qks, double num, double tauqks,
+                                       double dt) {
   constexpr double K = 0.28 * 0.28 * 0.28;
   const double c3 = csubt * csubt * csubt;
   const double d = c3 + K;
-  w.open(1);
-  w.put(0, dt * (0.2 * (d + num * c3) - qks * d), d * tauqks);
-  w.divide();
-  return w.get(0);
+  return Math<double>::div(dt * (0.2 * (d + num * c3) - qks * d), d * tauqks);
 }
 
 // Coefficients of the next lattice update for the FP32 lattice, computed in
@@ -538,21 +544,15 @@ __device__ inline double qks_increment_warp(double csubt, double qks, double num
 // 1 - dinf as exp(x) dinf, 1 - finf as the quotient it subtracts.  The flags
 // come from the FP64 fmods in fm (as step_coef_warp takes them) and the time
 // step constants from P.  Every lane returns the same coefficients.
-__device__ inline bool step_coef_warp_f32(StepCoef<float>& k, const rh_membrane& m,
-                                          const CellConst& c, double dt, const double* fm,
-                                          const MembranePre& P) {
+//
+// coef_voltage_f32 gives those that need the new voltage or [Na]i,
+// coef_known_f32 the rest (`t` the time of the next update).
+__device__ inline void coef_voltage_f32(StepCoef<float>& k, const CellConst& c, double vd,
+                                        double xnaid) {
   const int lane = threadIdx.x & 31;
-  const double vd = m.v;
-  const float v = (float)vd, xnai = (float)m.xnai;
-  float dv5 = 5.f, dvk = 8.f, fv5 = -22.8f, fvk = 9.1f;
-  k.alphac = 0.22f;
-  k.betac = 4.f;
-  if (c.iso2) {
-    k.betac = 2.f;
-    dv5 = 0.f;
-    fv5 = -28.f;
-    fvk = 8.5f;
-  }
+  const float v = (float)vd, xnai = (float)xnaid;
+  const float dv5 = c.iso2 ? 0.f : 5.f, dvk = 8.f;
+  const float fv5 = c.iso2 ? -28.f : -22.8f, fvk = c.iso2 ? 8.5f : 9.1f;
   const float za = v * (float)(FARAD / XRGAS / TEMPER);
   const float tq = 0.0337f * (v + 10.5f);
   // one exponential per lane: lanes 0-6 the arguments of step_coef
@@ -594,32 +594,46 @@ __device__ inline bool step_coef_warp_f32(StepCoef<float>& k, const rh_membrane&
   k.ncx_t1 = (float)(KMCAI * (XNAO * XNAO * XNAO)) * (1.f + r * r * r);
   k.ncx_t3a = (float)(KMCAO + c.cao) * xn3;
   k.ncx_den2 = 1.f + (float)KSAT * e2;
+  // build options (option_coef)
+  k.ncx_ka_hill = c.ncx_form == RH_NCX_OLD || (c.ncx_form == RH_NCX_NOALLO && vd < -75);
+  k.bcg_a = (float)(BCG_G * vd);
+}
+
+__device__ inline void coef_known_f32(StepCoef<float>& k, const CellConst& c, double t, double dt,
+                                      const double* fm, double rdt, double dth, double rdt95,
+                                      double rdth95) {
+  k.alphac = 0.22f;
+  k.betac = c.iso2 ? 2.f : 4.f;
   k.svica = (float)c.svica;
   k.svncx = (float)c.svncx;
   // build options (option_coef)
-  const double t = m.t;
   k.sviup = (float)((c.iso && t >= 5.5 * c.pcl) ? c.sviup_iso : c.sviup_tot);
   k.iso_add_lcc = c.iso && fm[4] < dt;
   k.ncx_form = c.ncx_form;
-  k.ncx_ka_hill = c.ncx_form == RH_NCX_OLD || (c.ncx_form == RH_NCX_NOALLO && vd < -75);
   k.ncx_t2b = (float)((KMNAI * KMNAI * KMNAI) * c.cao);
   k.slowncx = c.slowncx;
-  k.bcg_a = (float)(BCG_G * vd);
   k.bcg_b = (float)(BCG_G / 2. / FRT);
   k.cao = (float)c.cao;
   k.ku = (float)c.ku;
   k.ku2 = (float)c.ku2;
   k.kb = (float)c.kb;
   k.dt = (float)dt;
-  k.rdt = (float)P.rdt;
-  k.dth = (float)P.dth;
-  k.rdt95 = (float)P.rdt95;
-  k.rdth95 = (float)P.rdth95;
+  k.rdt = (float)rdt;
+  k.dth = (float)dth;
+  k.rdt95 = (float)rdt95;
+  k.rdth95 = (float)rdth95;
   k.reset_window = fm[0] < dt;
   k.output_step = fm[1] < dt;
   k.perm = c.perm;
   k.cadist_step = k.output_step && fm[2] < dt && fm[3] < 500;
-  return t < c.tend;
+}
+
+__device__ inline bool step_coef_warp_f32(StepCoef<float>& k, const rh_membrane& m,
+                                          const CellConst& c, double dt, const double* fm,
+                                          const MembranePre& P) {
+  coef_voltage_f32(k, c, m.v, m.xnai);
+  coef_known_f32(k, c, m.t, dt, fm, P.rdt, P.dth, P.rdt95, P.rdth95);
+  return m.t < c.tend;
 }
 
 }  // namespace rh

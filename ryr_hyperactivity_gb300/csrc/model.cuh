@@ -105,6 +105,11 @@ __device__ __forceinline__ bool extreme(double x) {
   return ((__double2hiint(x) + 0x00100000) & 0x7fe00000) == 0;
 }
 
+// Exponent field 0x7ff: infinite or NaN.
+__device__ __forceinline__ bool extreme_high(double x) {
+  return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000;
+}
+
 // Reciprocal of d from the hardware's rough reciprocal y0 (measured: off by
 // at most 2^-19.9) by one third-order step: with e = 1 - d y0, 1/d =
 // y0 (1 + e + e^2 + ...) and y0 (1 + e + e^2) is off by e^3 (Householder's
@@ -122,13 +127,16 @@ __device__ __forceinline__ double rcp_refine(double d, double y) {
 
 // a / b in six FP64 instructions: the reciprocal, the quotient and one
 // residual correction of it (equal to the rounded quotient in 39 million
-// random pairs).  A seed or quotient outside the normal range
-// takes the ordinary division.
+// random pairs).  A seed or quotient outside the normal range takes the
+// ordinary division, but for a zero numerator.
 __device__ __forceinline__ double div_refined(double a, double b) {
   const double y0 = rcp_seed(b);
   const double y = rcp_refine(b, y0);
-  const double q = a * y;
-  if (extreme(y0) || extreme(q)) return a / b;
+  const double q = __dmul_rn(a, y);
+  if (extreme(y0) || extreme(q)) {
+    const bool zero = ((__double2hiint(a) << 1) | __double2loint(a)) == 0;
+    return zero && !extreme(y0) ? q : a / b;
+  }
   return fma(fma(-b, q, a), y, q);
 }
 
@@ -204,9 +212,11 @@ __device__ __forceinline__ float2 vsub(float2 a, float2 b) {
   return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a);
 }
 __device__ __forceinline__ double2 vadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 vmul(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
+__device__ __forceinline__ double2 vmul(double2 a, double2 b) {
+  return make_double2(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y));
+}
 __device__ __forceinline__ double2 vfma(double2 a, double2 b, double2 c) {
-  return make_double2(a.x * b.x + c.x, a.y * b.y + c.y);
+  return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
 }
 __device__ __forceinline__ double2 vsub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 // x < 0 ? 0 : x, NaN staying NaN.  In FP32 one max.NaN instruction (its
@@ -278,14 +288,14 @@ __device__ __forceinline__ void serca_leak(double c, double n, double pa, double
   const double d = d1 * d2;
   const double y0 = rcp_seed(d);
   if (extreme(y0) || extreme(d1) || extreme(d2)) {
-    up = sviup * (nu / d1);
+    up = __dmul_rn(sviup, nu / d1);
     lk = nl / d2;
     return;
   }
   const double y = rcp_refine(d, y0);
   const double y1 = d2 * y, y2 = d1 * y;
   const double q1 = nu * y1, q2 = nl * y2;
-  up = sviup * fma(fma(-d1, q1, nu), y1, q1);
+  up = __dmul_rn(sviup, fma(fma(-d1, q1, nu), y1, q1));
   lk = fma(fma(-d2, q2, nl), y2, q2);
 }
 
@@ -294,6 +304,16 @@ __device__ __forceinline__ R pow23(R x) {  // x^23 = x^16 x^4 x^2 x
   R x2 = x * x, x4 = x2 * x2, x8 = x4 * x4, x16 = x8 * x8;
   return x16 * x4 * x2 * x;
 }
+
+// A product that branches of the build options may replace, before it is added
+// elsewhere.  FP64: rounded by itself, so that the kernel variants with and
+// without the options give the same bits whichever product the compiler would
+// fuse with the sum.
+__device__ __forceinline__ float own_product(float a, float b) { return a * b; }
+__device__ __forceinline__ double own_product(double a, double b) { return __dmul_rn(a, b); }
+// a b + c, fused in FP64 for the same reason.
+__device__ __forceinline__ float mad(float a, float b, float c) { return a * b + c; }
+__device__ __forceinline__ double mad(double a, double b, double c) { return fma(a, b, c); }
 
 // ---- buffers (buffers.c:55-155) ----
 
@@ -320,6 +340,7 @@ __device__ __forceinline__ R buffer_rate(R kon, R koff, R total, R bound, R c, R
                                          R rdt95) {
   R on = kon * c;
   on = saturates(on, dt, hr) ? rdt95 : on;
+  if constexpr (sizeof(R) == 8) return fma(on, total - bound, -__dmul_rn(koff, bound));
   return on * (total - bound) - koff * bound;
 }
 

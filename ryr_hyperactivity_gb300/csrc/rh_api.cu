@@ -340,6 +340,16 @@ StepArgs<R> make_args(rh_sim* s, const Lattice<R>& L, bool lattice_only) {
   return a;
 }
 
+// Whether the cell updates take four warps (cellwide.cuh): while the lattice
+// holds at most ten warps per SM, half of what an SM has room for, the cell
+// update is the step's critical path and its CTAs find room beside the
+// lattice's.  Four-warp against one-warp updates, per 100 steps: 50 cells of
+// 432 CRUs (5 warps per SM) 1.75 against 2.31 ms, 110 cells (10) 2.40 against
+// 2.46, 150 cells (14) 2.88 against 2.62.
+bool wide_cells(const rh_sim* s) {
+  return s->sets[kNarrowSet].ntiles <= 10 * (int64_t)s->sm_count;
+}
+
 // One group's step: the tiles of cells [group_cell[g], group_cell[g+1]),
 // then the whole-cell update of those cells.
 cudaError_t launch_group(rh_sim* s, int g, bool out, bool lattice_only, cudaStream_t st) {
@@ -355,7 +365,7 @@ cudaError_t launch_group(rh_sim* s, int g, bool out, bool lattice_only, cudaStre
     if ((e = launch_step<float>(a, te - tb, out, s->group_opt[g], t.tile, s->staging,
                                 &s->maps[s->ts], st)) != cudaSuccess)
       return e;
-    return launch_cells<float>(a, c0, c1 - c0, out, t.tile, st);
+    return launch_cells<float>(a, c0, c1 - c0, out, t.tile, wide_cells(s), st);
   }
   StepArgs<double> a = make_args(s, s->Ld, lattice_only);
   a.tiles += tb;
@@ -363,7 +373,7 @@ cudaError_t launch_group(rh_sim* s, int g, bool out, bool lattice_only, cudaStre
   if ((e = launch_step<double>(a, te - tb, out, s->group_opt[g], t.tile, 0, nullptr, st)) !=
       cudaSuccess)
     return e;
-  return launch_cells<double>(a, c0, c1 - c0, out, t.tile, st);
+  return launch_cells<double>(a, c0, c1 - c0, out, t.tile, wide_cells(s), st);
 }
 
 // The state of cells [c0, c1) between the device and a host image in the

@@ -20,14 +20,21 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "cellwide.cuh"
 #include "tile.cuh"
 
 namespace rh {
 
 template <class R, bool OUT>
 __global__ void __launch_bounds__(32, 16) cell_kernel(StepArgs<R> a, int cell0, int nw) {
-  __shared__ double scratch[160];
+  __shared__ double scratch[kCellScratch];
   cell_update<R, OUT, false>(a, cell0 + blockIdx.x, nw, scratch);
+}
+
+template <class R, bool OUT>
+__global__ void __launch_bounds__(kWideThreads) cell_wide_kernel(StepArgs<R> a, int cell0, int nw) {
+  __shared__ CellWideShared<R> sh;
+  cell_update_wide<R, OUT>(a, cell0 + blockIdx.x, nw, sh);
 }
 
 template <class R, bool OUT, int B, bool OPT, int STG>
@@ -203,12 +210,12 @@ cudaError_t launch_step(const StepArgs<R>& a, int ntiles, bool out, bool opt, in
 }
 
 template <class R>
-cudaError_t launch_cells(const StepArgs<R>& a, int cell0, int ncells, bool out, int tile,
+cudaError_t launch_cells(const StepArgs<R>& a, int cell0, int ncells, bool out, int tile, bool wide,
                          cudaStream_t st) {
   if (ncells <= 0) return cudaSuccess;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ncells);
-  cfg.blockDim = dim3(32);
+  cfg.blockDim = dim3(wide ? kWideThreads : 32);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = st;
   // Programmatic serialization after the lattice launch, and the device's
@@ -227,6 +234,9 @@ cudaError_t launch_cells(const StepArgs<R>& a, int cell0, int ncells, bool out, 
   cfg.attrs = at;
   cfg.numAttrs = 2;
   const int nw = tile / 32;
+  if (wide)
+    return out ? cudaLaunchKernelEx(&cfg, cell_wide_kernel<R, true>, a, cell0, nw)
+               : cudaLaunchKernelEx(&cfg, cell_wide_kernel<R, false>, a, cell0, nw);
   if (out) return cudaLaunchKernelEx(&cfg, cell_kernel<R, true>, a, cell0, nw);
   return cudaLaunchKernelEx(&cfg, cell_kernel<R, false>, a, cell0, nw);
 }
@@ -250,9 +260,9 @@ template cudaError_t launch_step<double>(const StepArgs<double>&, int, bool, boo
                                          const StageMaps*, cudaStream_t);
 template cudaError_t launch_step<float>(const StepArgs<float>&, int, bool, bool, int, int,
                                         const StageMaps*, cudaStream_t);
-template cudaError_t launch_cells<double>(const StepArgs<double>&, int, int, bool, int,
+template cudaError_t launch_cells<double>(const StepArgs<double>&, int, int, bool, int, bool,
                                           cudaStream_t);
-template cudaError_t launch_cells<float>(const StepArgs<float>&, int, int, bool, int,
+template cudaError_t launch_cells<float>(const StepArgs<float>&, int, int, bool, int, bool,
                                          cudaStream_t);
 template cudaError_t launch_init<double>(const Lattice<double>&, const CellConst*,
                                          const InitValues*, int, int, cudaStream_t);

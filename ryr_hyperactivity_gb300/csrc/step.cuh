@@ -106,9 +106,10 @@ cudaError_t launch_step(const StepArgs<R>& a, int ntiles, bool out, bool opt, in
                         int staging, const StageMaps* maps, cudaStream_t st);
 
 // The whole-cell update of cells [cell0, cell0 + ncells) after their lattice
-// launch on the same stream (`tile` is the lattice launch's tile length).
+// launch on the same stream (`tile` is the lattice launch's tile length), by
+// one warp per cell or, `wide`, by four (cellwide.cuh).
 template <class R>
-cudaError_t launch_cells(const StepArgs<R>& a, int cell0, int ncells, bool out, int tile,
+cudaError_t launch_cells(const StepArgs<R>& a, int cell0, int ncells, bool out, int tile, bool wide,
                          cudaStream_t st);
 
 // Whether a cell's lattice update uses any build option of the `opt` variant.

@@ -62,13 +62,14 @@ __device__ __forceinline__ void wait_for_prerequisite_grid() {
 // microseconds of dependent FP64 latency on this GPU) out of the lattice
 // CTAs; at <= 128 registers a cell warp fits beside five lattice CTAs.
 // `nw` is the number of warps per lattice tile (the rows of output partials
-// each tile wrote).
+// each tile wrote); `scratch` is kCellScratch doubles of shared memory.
 //
 // The same update runs inside the persistent window kernel (PERSIST), by one
 // warp of a CTA that takes the cell's update from the queue: there is no
 // prior launch to wait for, the output step is the cell's own flag (OUT =
 // true reads it), and a device-scope fence first makes the cell's state,
 // written by other CTAs during the launch, visible to the warp's loads.
+constexpr int kCellScratch = 160 + NOUT;
 template <class R, bool OUT, bool PERSIST>
 __device__ __forceinline__ void cell_update(const StepArgs<R>& a, int cell, int nw,
                                             double* scratch) {
@@ -90,30 +91,15 @@ __device__ __forceinline__ void cell_update(const StepArgs<R>& a, int cell, int 
   if (!PERSIST) wait_for_prerequisite_grid();
 
   if (!a.lattice_only) {
-    const double* P = a.partials;
-    // output-step partials: one row per warp of each of the cell's tiles
-    const int t0 = cc.tile_begin * nw, nt = cc.tile_count * nw;
     // the step's exact whole-cell sums, accumulated by the cell's CTAs
     double tot[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q)
       tot[q] = fx_to_double(__ldcg(&dyn->acc[2 * q]), __ldcg(&dyn->acc[2 * q + 1]));
-    double osum[NOUT];
-    if (out_step) {
-      for (int q = 0; q < NOUT; ++q) {
-        double s = 0.0;
-        for (int tl = lane; tl < nt; tl += 32)
-          s += __ldcg(P + (size_t)(t0 + tl) * P_COUNT + P_STEP_END + q);
-        osum[q] = warp_sum(s);
-      }
-      // the ci > 1000 flag is a max, not a sum
-      double f = 0.0;
-      for (int tl = lane; tl < nt; tl += 32)
-        f = fmax(f, __ldcg(P + (size_t)(t0 + tl) * P_COUNT + O_CIHIGH));
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) f = fmax(f, __shfl_down_sync(0xffffffffu, f, off));
-      osum[O_CIHIGH - P_STEP_END] = f;
-    }
+    double* osum = scratch + 160;  // [NOUT]
+    if (out_step)
+      output_sums_warp(a.partials + (size_t)cc.tile_begin * nw * P_COUNT, cc.tile_count * nw, osum,
+                       lane);
     // reduction quotients, [Na]i and V (:447-456, :701-738)
     membrane_post_warp(m, dt, cc, tot, scratch, pre);
     uint32_t status = __ldcg(&dyn->status);
@@ -134,9 +120,19 @@ __device__ __forceinline__ void cell_update(const StepArgs<R>& a, int cell, int 
       active = step_coef_warp(kd, m, cc, dt, fm + 1, scratch, &qs);
       m.qks = m.qks + qs.dqks;
     } else {
-      const double dqks = qks_increment_warp(m.csubt, m.qks, pre.qks_num, pre.tauqks, dt, scratch);
+      const double dqks = qks_increment(m.csubt, m.qks, pre.qks_num, pre.tauqks, dt);
       active = step_coef_warp_f32(kf, m, cc, dt, fm + 1, pre);
       m.qks = m.qks + dqks;
+    }
+    double* w = nullptr;
+    if (out_step) {
+      m.sparksum += (long long)osum[O_SPARK - P_STEP_END];
+      if (osum[O_CIHIGH - P_STEP_END] > 0) status |= RH_STATUS_CI_HIGH;
+      w = a.out_wc + ((size_t)cell * a.out_cap + dyn->out_count % a.out_cap) * RH_WHOLECELL_COLS;
+      const double t_next = m.t;
+      m.t = t_step;
+      wholecell_columns_warp(w, osum, m, cc.n, dt, lane);
+      m.t = t_next;
     }
     if (lane == 0) {
       if (a.stats) {  // per-beat detectors on the (t, V) sample of this step
@@ -147,14 +143,6 @@ __device__ __forceinline__ void cell_update(const StepArgs<R>& a, int cell, int 
         }
       }
       if (out_step) {
-        m.sparksum += (long long)osum[O_SPARK - P_STEP_END];
-        if (osum[O_CIHIGH - P_STEP_END] > 0) status |= RH_STATUS_CI_HIGH;
-        long long slot = dyn->out_count % a.out_cap;
-        double* w = a.out_wc + ((size_t)cell * a.out_cap + slot) * RH_WHOLECELL_COLS;
-        const double t_next = m.t;
-        m.t = t_step;
-        wholecell_columns(w, osum, m, cc.n, dt);
-        m.t = t_next;
         if (cadist) {  // record header: t and V of this output step (:1005)
           double* h = a.out_cd + cc.cd_off + (dyn->cd_count % a.cd_cap) * (2 + 6 * (long long)cc.n);
           h[0] = t_step;
@@ -603,8 +591,8 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
     const R cn0 = s_cn2[0][tid].x, cn1 = s_cn2[0][tid].y;
     const R diffpi0 = (cp - ci0) * R(1.0 / TAUPI / 2.);
     const R diffpi1 = (cp - ci1) * R(1.0 / TAUPI / 2.);
-    const R diffsi0 = (cs0 - ci0) * R(1.0 / TAUSI / 2.);
-    const R diffsi1 = (cs0 - ci1) * R(1.0 / TAUSI / 2.);
+    const R diffsi0 = own_product(cs0 - ci0, R(1.0 / TAUSI / 2.));
+    const R diffsi1 = own_product(cs0 - ci1, R(1.0 / TAUSI / 2.));
     const R diffjn0 = (cjsr - cn0) * R(1.0 / TAUTR / 2.);
     const R diffjn1 = (cjsr - cn1) * R(1.0 / TAUTR / 2.);
 
@@ -670,7 +658,7 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
     if (!o_perm) {
       R ica = k.lcc_k * (cpx * k.lcc_e2z_k - k.cao);
       if (ica > R(0)) ica = R(0);
-      icat1 = k.svica * R(nlcp) * ica;
+      icat1 = own_product(k.svica * R(nlcp), ica);
     }
 
     // ---- RyR gating, spark flag, release (:1274-1293) ----
@@ -697,7 +685,7 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
                                      (k.ncx_t1 + t2 + t3) * k.ncx_den2);
         const R r3 = Math<R>::div(R(0.0003), csm);
         ancx += (Math<R>::div(R(1), R(1) + r3 * r3 * r3) - ancx) * R(1.0 / 150.) * dt;
-        xinaca = k.svncx * inaca;
+        xinaca = own_product(k.svncx, inaca);
       } else {  // oldncx (:77-100) and ncx_noallo (:102-120)
         R ka = R(1);
         if (k.ncx_ka_hill) {
@@ -714,7 +702,7 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
           if (on * dt > R(0.95)) da = k.rdt95 * (R(1) - ancx) - ancx * R(KNCXOFF_OLD);
           ancx += da * dt;
         }
-        xinaca = k.svncx * inaca;
+        xinaca = own_product(k.svncx, inaca);
       }
     }
     // slowncxchange background Ca current (:1267-1269), into xicat and the
@@ -741,10 +729,14 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
       R csN = cs_face, csS = cs_face;
       if (has_zp) csN = BULK ? b_hcs[1][tid + ocp] : kStage ? s_hcs[1][tid] : __ldg(cs + g + lxly);
       if (has_zm) csS = BULK ? b_hcs[0][tid + ocm] : kStage ? s_hcs[0][tid] : __ldg(cs + g - lxly);
-      const R csdiff = (csN + csS - R(2) * cs0) * R(1.0 / TAUST);
-      const R cs_const = -R(ICAGAMMA * VP / VS) * icat1 + xinaca -
-                         (cs0 - ci0) * R(1.0 / TAUSI / 2.) - (cs0 - ci1) * R(1.0 / TAUSI / 2.) +
-                         csdiff - bcgcur;
+      const R csdiff = own_product(csN + csS - R(2) * cs0, R(1.0 / TAUST));
+      R cs_const;
+      if constexpr (sizeof(R) == 8)
+        cs_const = -R(ICAGAMMA * VP / VS) * icat1 + xinaca - diffsi0 - diffsi1 + csdiff - bcgcur;
+      else
+        cs_const = -R(ICAGAMMA * VP / VS) * icat1 + xinaca -
+                   (cs0 - ci0) * R(1.0 / TAUSI / 2.) - (cs0 - ci1) * R(1.0 / TAUSI / 2.) +
+                   csdiff - bcgcur;
       const R cp_const =
           (ci0 - cp) * R(1.0 / TAUPI / 2.) + (ci1 - cp) * R(1.0 / TAUPI / 2.) + xire - icat1;
 #pragma unroll 1
@@ -752,18 +744,18 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
         const R r_sar = buffer_rate<R>(R(KSARON), R(KSAROFF), R(BSAR), casar, csn, dth, hrh, rdth95);
         const R r_sarh =
             buffer_rate<R>(R(KSARHON), R(KSARHOFF), R(BSARH), casarh, csn, dth, hrh, rdth95);
-        R dotcs = R(VP / VS / TAUPS) * (cp - csn) + cs_const - (r_sar + r_sarh);
+        R dotcs = mad(R(VP / VS / TAUPS), cp - csn, cs_const) - (r_sar + r_sarh);
         if (o_perm) dotcs += (R(PERM_CI_BASAL) - csn) * R(0.2);  // :1409-1411
         const R cpbuff = buffer_rate<R>(R(KSARON), R(KSAROFF), R(BSAR), casarj, cp, dth, hrh, rdth95);
         const R cpbuffh =
             buffer_rate<R>(R(KSARHON), R(KSARHOFF), R(BSARH), casarhj, cp, dth, hrh, rdth95);
-        const R cpdot = (csn - cp) * R(1.0 / TAUPS) + cp_const - cpbuff - cpbuffh;
-        casarj = clamp0(casarj + cpbuff * dth);
-        casarhj = clamp0(casarhj + cpbuffh * dth);
-        cp += cpdot * dth;
-        casar = clamp0(casar + r_sar * dth);
-        casarh = clamp0(casarh + r_sarh * dth);
-        csn += dotcs * dth;
+        const R cpdot = mad(csn - cp, R(1.0 / TAUPS), cp_const) - cpbuff - cpbuffh;
+        casarj = clamp0(mad(cpbuff, dth, casarj));
+        casarhj = clamp0(mad(cpbuffh, dth, casarhj));
+        cp = mad(cpdot, dth, cp);
+        casar = clamp0(mad(r_sar, dth, casar));
+        casarh = clamp0(mad(r_sarh, dth, casarh));
+        csn = mad(dotcs, dth, csn);
       }
     }
     cp = clamp0(cp);
@@ -942,12 +934,21 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
         cix_ex = ci_ex;
         cnx_ex = cn_ex;
       }
-      const V coupn =
-          vfma(vadd(vadd(vadd(vsub(cnN, n), vsub(cnS, n)), vsub(cny_in, n)), vsub(cny_ex, n)), kt_n,
-               vmul(vadd(vsub(cnx_in, n), vsub(cnx_ex, n)), kl_n));
-      const V coupi =
-          vfma(vadd(vadd(vadd(vsub(ciN, c), vsub(ciS, c)), vsub(ciy_in, c)), vsub(ciy_ex, c)), kt_i,
-               vmul(vadd(vsub(cix_in, c), vsub(cix_ex, c)), kl_i));
+      // sums of the pair's differences along z: the halves' own difference
+      // enters both with opposite signs, which saves an FP64 subtraction
+      V cnz, ciz;
+      if constexpr (sizeof(R) == 8) {
+        const R dn = n.y - n.x, dc = c.y - c.x;
+        cnz = v2(dn + (cnS.x - n.x), (cnN.y - n.y) - dn);
+        ciz = v2(dc + (ciS.x - c.x), (ciN.y - c.y) - dc);
+      } else {
+        cnz = vadd(vsub(cnN, n), vsub(cnS, n));
+        ciz = vadd(vsub(ciN, c), vsub(ciS, c));
+      }
+      const V coupn = vfma(vadd(vadd(cnz, vsub(cny_in, n)), vsub(cny_ex, n)), kt_n,
+                           vmul(vadd(vsub(cnx_in, n), vsub(cnx_ex, n)), kl_n));
+      const V coupi = vfma(vadd(vadd(ciz, vsub(ciy_in, c)), vsub(ciy_ex, c)), kt_i,
+                           vmul(vadd(vsub(cix_in, c), vsub(cix_ex, c)), kl_i));
       // SERCA and leak (subroutine_cuda.c:128-146)
       V up, lk;
       {
@@ -999,8 +1000,10 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
           sr = buffer_rate<R>(R(KSRON), R(KSROFF), R(BSR), h ? casr.y : casr.x, cv, dt, hr, k.rdt95);
         }
       }
-      V dotcn = vfma(vsub(up, lk), splat2(R(VI / VNSR)), coupn);
-      V dotci = vadd(vsub(vsub(lk, up), vadd(vadd(vadd(vadd(r_tf, r_ts), r_cal), r_sr), r_mc)), coupi);
+      const V net = vsub(up, lk);
+      V dotcn = vfma(net, splat2(R(VI / VNSR)), coupn);
+      // coupi - (up - lk) - sum of the buffer rates
+      V dotci = vsub(coupi, vadd(net, vadd(vadd(vadd(vadd(r_tf, r_ts), r_cal), r_sr), r_mc)));
       if (p == 0) {  // sub-voxels 0 and 1 touch the dyad, submembrane and JSR (:1356-1361)
         dotcn = vfma(v2(diffjn0, diffjn1), splat2(R(VJSR / VNSR)), dotcn);
         dotci = vfma(v2(diffsi0, diffsi1), splat2(R(VS / VI)), dotci);

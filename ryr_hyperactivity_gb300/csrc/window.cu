@@ -191,7 +191,7 @@ template <class R, int B, bool OPT, int MINB>
 __global__ void __launch_bounds__(B, MINB) window_kernel(StepArgs<R> a, WindowCtl w) {
   __shared__ TileHeader sh;
   __shared__ StepCoef<R> sk;
-  __shared__ double scratch[160];
+  __shared__ double scratch[kCellScratch];
   __shared__ StepArgs<R> s_a;  // arguments of the out-of-line cold paths
   __shared__ WindowCtl s_w;
   __shared__ int s_go[2];
