@@ -303,19 +303,18 @@ bool use_persist(const rh_sim* s) {
 }
 
 // The tile table the two-launch path runs: the launch shape's, or the narrow
-// tiles (one warp per CTA) where no shape was asked for and one wave of warps
-// holds the whole lattice.  128-CRU tiles then leave SMs without work: a
-// 100x20x10 cell fills 111 of 152.  FP64, up to the 12 warps an SM holds (a
-// warp's rate is set by its scheduler's FP64 unit, so warps want spreading):
-// per 100 steps, one 20x10x5 cell 6.39 ms against 6.57, one 100x20x10 cell
-// 7.06 against 7.40, ten 3,705-CRU cells 10.16 against 10.75.  FP32, up to one
-// warp per scheduler: one 100x20x10 cell 2.33 against 2.37 ms, but 200 cells of
-// 432 CRUs (18 warps per SM) 3.68 against 2.91: four-warp CTAs share their
-// header, staging and barriers.
+// tiles (32 CRUs per CTA) where no shape was asked for and the lattice is
+// small.  128-CRU tiles then leave SMs without work: a 100x20x10 cell fills
+// 111 of 152.  FP64, up to 12 tiles per SM, the warps an SM holds: a warp's
+// rate is set by its scheduler's FP64 unit, so warps want spreading (per 100
+// steps: 1,350 tiles 10.1 ms, but 2,700 tiles 19.9 ms against 19.2 with the
+// default).  FP32, up to the three split tiles an SM holds (narrow against
+// default tiles: one 100x20x10 cell 1.51 against 1.58 ms, two 80x16x8 cells
+// 1.40 against 1.44, 35 cells of 432 CRUs (490 tiles) 1.89 against 1.68).
 int active_set(const rh_sim* s) {
   if (s->shape_given || use_persist(s)) return s->ts;
-  const int64_t warps_per_sm = is_mixed(s) ? 4 : 12;
-  return s->sets[kNarrowSet].ntiles <= warps_per_sm * s->sm_count ? kNarrowSet : s->ts;
+  const int64_t tiles_per_sm = is_mixed(s) ? kSplitBlocks : 12;
+  return s->sets[kNarrowSet].ntiles <= tiles_per_sm * s->sm_count ? kNarrowSet : s->ts;
 }
 
 template <class R>
@@ -350,6 +349,15 @@ bool wide_cells(const rh_sim* s) {
   return s->sets[kNarrowSet].ntiles <= 10 * (int64_t)s->sm_count;
 }
 
+// Whether the narrow tiles are split over five warps (tile.cuh).  Only one
+// cell group in a second, mostly empty wave prefers one warp per tile (552
+// tiles of one FP64 cell: 6.90 against 7.37 ms per 100 steps); other groups'
+// tiles fill such a wave (540 tiles of two cells: split 5.61 against 6.69).
+bool split_tiles(const rh_sim* s) {
+  const int64_t tiles = s->sets[kNarrowSet].ntiles, wave = (int64_t)kSplitBlocks * s->sm_count;
+  return active_set(s) == kNarrowSet && (s->ngroups > 1 || tiles <= wave || tiles >= 2 * wave);
+}
+
 // One group's step: the tiles of cells [group_cell[g], group_cell[g+1]),
 // then the whole-cell update of those cells.
 cudaError_t launch_group(rh_sim* s, int g, bool out, bool lattice_only, cudaStream_t st) {
@@ -362,7 +370,8 @@ cudaError_t launch_group(rh_sim* s, int g, bool out, bool lattice_only, cudaStre
     StepArgs<float> a = make_args(s, s->Lf, lattice_only);
     a.tiles += tb;
     a.tile_base = tb;
-    if ((e = launch_step<float>(a, te - tb, out, s->group_opt[g], t.tile, s->staging,
+    if ((e = launch_step<float>(a, te - tb, out, s->group_opt[g], t.tile,
+                                split_tiles(s) ? 3 : s->staging,
                                 &s->maps[s->ts], st)) != cudaSuccess)
       return e;
     return launch_cells<float>(a, c0, c1 - c0, out, t.tile, wide_cells(s), st);
@@ -370,8 +379,8 @@ cudaError_t launch_group(rh_sim* s, int g, bool out, bool lattice_only, cudaStre
   StepArgs<double> a = make_args(s, s->Ld, lattice_only);
   a.tiles += tb;
   a.tile_base = tb;
-  if ((e = launch_step<double>(a, te - tb, out, s->group_opt[g], t.tile, 0, nullptr, st)) !=
-      cudaSuccess)
+  if ((e = launch_step<double>(a, te - tb, out, s->group_opt[g], t.tile, split_tiles(s) ? 3 : 0,
+                               nullptr, st)) != cudaSuccess)
     return e;
   return launch_cells<double>(a, c0, c1 - c0, out, t.tile, wide_cells(s), st);
 }

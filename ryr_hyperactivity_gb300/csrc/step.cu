@@ -38,7 +38,8 @@ __global__ void __launch_bounds__(kWideThreads) cell_wide_kernel(StepArgs<R> a, 
 }
 
 template <class R, bool OUT, int B, bool OPT, int STG>
-__global__ void __launch_bounds__(B, min_blocks_for<R, B>())
+__global__ void __launch_bounds__(STG == 3 ? 32 * kSplitWarps : B,
+                                  STG == 3 ? kSplitBlocks : min_blocks_for<R, B>())
     step_kernel(StepArgs<R> a, const __grid_constant__ StageMaps maps) {
   __shared__ TileHeader sh;
   __shared__ StepCoef<R> sk;
@@ -46,7 +47,7 @@ __global__ void __launch_bounds__(B, min_blocks_for<R, B>())
   __shared__ __align__(8) uint64_t bars[2];
   extern __shared__ __align__(128) unsigned char dsm[];  // tensor copies land 128-byte aligned
   allow_dependent_launch();  // the cell update may start its first part
-  if (STG != 0 && threadIdx.x == 0) {  // ordered before the other threads' waits by the header barrier
+  if ((STG == 1 || STG == 2) && threadIdx.x == 0) {  // ordered before the other threads' waits by the header barrier
     mbar_init(&bars[0], 1);
     mbar_init(&bars[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -164,13 +165,14 @@ cudaError_t prepare_step_kernels() {
 template <class R, int B, int STG>
 void launch_bb(const StepArgs<R>& a, const StageMaps& maps, int ntiles, bool out, bool opt,
                cudaStream_t st) {
-  constexpr size_t smem = STG == 1 ? TileSmem<R, B>::kBytesBulk : TileSmem<R, B>::kBytes;
+  constexpr size_t smem = STG == 1 ? TileSmem<R, B>::kBytesBulk : TileSmem<R, B, STG == 3>::kBytes;
+  constexpr int T = STG == 3 ? 32 * kSplitWarps : B;
   if (opt) {
-    if (out) step_kernel<R, true, B, true, STG><<<ntiles, B, smem, st>>>(a, maps);
-    else step_kernel<R, false, B, true, STG><<<ntiles, B, smem, st>>>(a, maps);
+    if (out) step_kernel<R, true, B, true, STG><<<ntiles, T, smem, st>>>(a, maps);
+    else step_kernel<R, false, B, true, STG><<<ntiles, T, smem, st>>>(a, maps);
   } else {
-    if (out) step_kernel<R, true, B, false, STG><<<ntiles, B, smem, st>>>(a, maps);
-    else step_kernel<R, false, B, false, STG><<<ntiles, B, smem, st>>>(a, maps);
+    if (out) step_kernel<R, true, B, false, STG><<<ntiles, T, smem, st>>>(a, maps);
+    else step_kernel<R, false, B, false, STG><<<ntiles, T, smem, st>>>(a, maps);
   }
 }
 
@@ -200,7 +202,10 @@ cudaError_t launch_step(const StepArgs<R>& a, int ntiles, bool out, bool opt, in
   static const StageMaps kNoMaps{};
   const StageMaps& m = maps ? *maps : kNoMaps;
   switch (tile) {
-    case kNarrowTile: launch_bb<R, kNarrowTile, 0>(a, m, ntiles, out, opt, st); break;
+    case kNarrowTile:
+      if (staging == 3) launch_bb<R, kNarrowTile, 3>(a, m, ntiles, out, opt, st);
+      else launch_bb<R, kNarrowTile, 0>(a, m, ntiles, out, opt, st);
+      break;
     case 64: launch_b<R, 64>(a, m, ntiles, out, opt, staging, st); break;
     case 128: launch_b<R, 128>(a, m, ntiles, out, opt, staging, st); break;
     case 256: launch_b<R, 256>(a, m, ntiles, out, opt, staging, st); break;

@@ -13,9 +13,10 @@ constexpr int kNumTileSizes = 3;
 constexpr int kTileSizes[kNumTileSizes] = {64, 128, 256};
 constexpr int kDefaultTile = 128;
 
-// Narrow tiles, one warp per CTA, which the library uses by itself (they are
-// no launch shape) where the default tiles would leave SMs idle or unevenly
-// loaded; the simulator keeps their tile table after the kTileSizes ones.
+// Narrow tiles, one or five warps per CTA, which the library uses by itself
+// (they are no launch shape) where the default tiles would leave SMs idle or
+// unevenly loaded; the simulator keeps their tile table after the kTileSizes
+// ones.
 constexpr int kNarrowTile = 32;
 constexpr int kNarrowSet = kNumTileSizes;
 constexpr int kNumTileSets = kNumTileSizes + 1;
@@ -37,6 +38,9 @@ __host__ __device__ constexpr int min_blocks_for() {
   return sizeof(R) == 4 ? (B == 32 ? 20 : B == 64 ? 10 : (B == 128 ? 5 : 2))
                         : (B == 32 ? 12 : B == 64 ? 6 : (B == 128 ? 3 : 1));
 }
+
+// CTAs of a split tile (five warps, tile.cuh) an SM is to hold.
+constexpr int kSplitBlocks = 3;
 
 // Basal values of one cell (Init kernel, cuda_Cell_Detailed.cu:1121-1174),
 // computed on the host in FP64 and broadcast to every CRU of the cell.
@@ -95,7 +99,7 @@ template <class R>
 cudaError_t window_grid(int tile, bool opt, bool fewer_ctas, int* ctas);
 
 // One time step with tiles of `tile` CRUs (one of kTileSizes, or kNarrowTile
-// with staging 0).  `opt` selects
+// with staging 0, or 3 for split tiles).  `opt` selects
 // the kernel variant that handles the per-cell build options of the lattice
 // update (perm, iso, slowncxchange, NCX form); without them a cell runs the
 // plain variant.

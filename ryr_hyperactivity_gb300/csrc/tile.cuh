@@ -176,6 +176,22 @@ __device__ __forceinline__ void cell_update(const StepArgs<R>& a, int cell, int 
 
 // ------------------------------------------------------------- step kernel
 
+// Split tiles (STG 3, 32 CRUs): five warps share a tile, lane = CRU.  Four
+// take one z-pair of sub-voxels each, one the channel part; both parts read
+// only the old state, so nothing passes between the warps but the output
+// step's per-pair sums.  For lattices too small to fill the GPU, where a
+// step takes as long as one warp's instructions: in FP64 a warp issues one
+// FP64 instruction every 64 cycles, 1,170 of them for a whole tile, 420 at
+// most on any of the SM's four schedulers when split.  100 steps of one cell,
+// one warp per tile and split: 20x10x5 FP64 5.90 and 2.82 ms, 100x20x10 FP64
+// 6.40 and 5.30, 100x20x10 mixed 1.62 and 1.51.
+constexpr int kSplitWarps = 5;
+constexpr int kChannelWarp = 3;  // the pairs 0-3 are warps 0, 1, 2, 4
+// output-step sums of a pair and the statistics they belong to
+constexpr int kPairSums = 10;
+__device__ constexpr int kPairSumOf[kPairSums] = {O_CNSR, O_CI, O_CATF, O_CATS, O_CASR,
+                                                  O_CAMYO, O_CACAL, O_LEAK, O_UP, O_CIHIGH};
+
 // Dynamic shared memory of one CTA (tile of B CRUs).  Always the z-pair
 // planes of ci and cnsr, which the stencil reads from neighbouring threads.
 // FP32 kernels also stage, with asynchronous copies issued at the top of the
@@ -184,10 +200,10 @@ __device__ __forceinline__ void cell_update(const StepArgs<R>& a, int cell, int 
 // along y and z, and one CRU at each end along x), so the sub-voxel loop
 // reads no neighbour from global memory.  The FP64 kernels are bound by the
 // FP64 pipe, not by memory latency, and read global memory directly.
-template <class R, int B>
+template <class R, int B, bool SPLIT = false>
 struct TileSmem {
   using V = typename Vec2<R>::T;
-  static constexpr bool kStage = sizeof(R) == 4;
+  static constexpr bool kStage = sizeof(R) == 4 && !SPLIT;
   // The six cytosolic buffer fields (half of the state) are read straight
   // from global memory inside the sub-voxel loop: staging them as well costs
   // more in resident CTAs than it saves in latency.
@@ -209,7 +225,11 @@ struct TileSmem {
   static constexpr size_t kHz = kHy + 8 * kPlane;
   static constexpr size_t kHcs = kHz + 16 * sizeof(R) * B;  // R[dir][B]
   static constexpr size_t kHx = kHcs + 2 * sizeof(R) * B;  // V[2][4][2]
-  static constexpr size_t kBytes = kStage ? kHx + 16 * sizeof(V) : 8 * kPlane;
+  // split tiles: the pair warps' output-step sums, R[pair][kPairSums][B]
+  static constexpr size_t kSums = 8 * kPlane;
+  static constexpr size_t kBytes = SPLIT    ? kSums + 4 * kPairSums * sizeof(R) * B
+                                   : kStage ? kHx + 16 * sizeof(V)
+                                            : 8 * kPlane;
   // The bulk-copy staging (BULK, FP32 only) keeps the tile's own planes,
   // scalars and integers at the offsets above and moves the halo as whole
   // rows: each of the y and z halo planes holds B + 2 pairs (the row may
@@ -312,17 +332,21 @@ struct TileHeader {
 //   2: thread 0 issues 2-D tensor copies (cp.async.bulk.tensor, `maps`) of the
 //      tile's eight per-CRU real planes (bars[0], before the cell header
 //      arrives) and of its ci and cnsr pair planes (bars[1]); the integers,
-//      cs and the halo stay per-thread copies as in 0.
+//      cs and the halo stay per-thread copies as in 0;
+//   3: split tile (both precisions): kSplitWarps warps, no staging beyond the
+//      own pair planes.
 template <class R, bool OUT, int B, bool OPT, int STG = 0>
 __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHeader& sh,
                                             StepCoef<R>& sk, unsigned char* dsm,
                                             uint64_t* bars = nullptr, uint32_t phase = 0,
                                             const StageMaps* maps = nullptr) {
   constexpr int kBlock = B;
-  using TS = TileSmem<R, B>;
+  constexpr bool SPLIT = STG == 3;
+  using TS = TileSmem<R, B, SPLIT>;
   constexpr bool kStage = TS::kStage;
   constexpr bool BULK = STG == 1, TMA = STG == 2;
-  static_assert(STG == 0 || kStage, "bulk and tensor staging are the FP32 staging");
+  static_assert(STG == 0 || SPLIT || kStage, "bulk and tensor staging are the FP32 staging");
+  static_assert(!SPLIT || B == 32, "one CRU per lane");
   using V = typename Vec2<R>::T;
   V(*s_ci2)[kBlock] = reinterpret_cast<V(*)[kBlock]>(dsm + TS::kCi);
   V(*s_cn2)[kBlock] = reinterpret_cast<V(*)[kBlock]>(dsm + TS::kCn);
@@ -336,10 +360,16 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
   R(*s_hz)[4][2][kBlock] = reinterpret_cast<R(*)[4][2][kBlock]>(dsm + TS::kHz);
   R(*s_hcs)[kBlock] = reinterpret_cast<R(*)[kBlock]>(dsm + TS::kHcs);
   V(*s_hx)[4][2] = reinterpret_cast<V(*)[4][2]>(dsm + TS::kHx);
+  R(*s_sum)[kPairSums][kBlock] = reinterpret_cast<R(*)[kPairSums][kBlock]>(dsm + TS::kSums);
 
   const int4 tile = a.tiles[ti];
   const int cell = tile.x;
-  const int tid = threadIdx.x;
+  // the thread's CRU within the tile; split tiles: its warp's pair, or -1 for
+  // the channel part
+  const int tid = SPLIT ? (int)threadIdx.x & 31 : (int)threadIdx.x;
+  const int wid = (int)threadIdx.x >> 5;
+  const int pair = !SPLIT ? 0 : wid < kChannelWarp ? wid : wid == kChannelWarp ? -1 : 3;
+  const bool channel = !SPLIT || pair < 0, subs = !SPLIT || pair >= 0;
   const int cpad = (tile.z + 31) & ~31;  // cells are padded to 32 CRUs
   // Arena indices are 32-bit: the arena holds fewer than 2^29 CRUs (checked at
   // creation), so every element index, 8 sub-voxels per CRU included, is
@@ -378,8 +408,9 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
     const CellDyn* d = a.dyn + cell;
     const int* src = reinterpret_cast<const int*>(coef_ptr<R>(d));
     int* dst = reinterpret_cast<int*>(&sk);
-    for (int w = tid; w < (int)(sizeof(StepCoef<R>) / 4); w += blockDim.x) dst[w] = __ldcg(src + w);
-    if (tid == 0) {
+    for (int w = threadIdx.x; w < (int)(sizeof(StepCoef<R>) / 4); w += blockDim.x)
+      dst[w] = __ldcg(src + w);
+    if (threadIdx.x == 0) {
       const CellConst& c = a.cells[cell];
       sh.lx = c.lx;
       sh.ly = c.ly;
@@ -497,6 +528,7 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
   }
 
   // ---- stage the tile's own sub-voxels (z-pairs) ----
+  R old_cp = R(0), old_cjsr = R(0);  // split tiles, pair 0
   if (kStage && !BULK) {
     constexpr int kTpp = kBlock / 2;
     const int c2 = tid % kTpp, h2 = tid / kTpp;
@@ -550,6 +582,15 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
     cp_async_wait_group<1>();  // group 1 has landed (this thread's part of it)
     if (TMA && !(mbar_wait(&bars[0], phase) && mbar_wait(&bars[1], phase)))
       atomicOr(&a.dyn[cell].status, (unsigned int)RH_STATUS_TIMEOUT);
+  } else if (SPLIT) {
+    if (subs) {
+      s_ci2[pair][tid] = valid ? ci2[pair * S + g] : splat2(R(0));
+      s_cn2[pair][tid] = valid ? cn2[pair * S + g] : splat2(R(0));
+    }
+    if (valid && pair == 0) {  // read before the channel warp updates them
+      old_cp = L.cp[g];
+      old_cjsr = L.cjsr[g];
+    }
   } else if (!kStage) {
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
@@ -584,7 +625,12 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
     V* cnnext2 = reinterpret_cast<V*>(L.cnsr[par ^ 1]);
     R* csnext = L.cs[par ^ 1];
 
-    R cp = kSS ? s_sc[0][tid] : L.cp[g], cjsr = kSS ? s_sc[1][tid] : L.cjsr[g];
+    R cp, cjsr;
+    if (SPLIT && !channel) {
+      cp = old_cp, cjsr = old_cjsr;
+    } else {
+      cp = kSS ? s_sc[0][tid] : L.cp[g], cjsr = kSS ? s_sc[1][tid] : L.cjsr[g];
+    }
     const R cs0 = kStage ? s_cs[tid] : cs[g];
     // ---- dyad/submembrane/JSR coupling terms from the old state (:1309-1314) ----
     const R ci0 = s_ci2[0][tid].x, ci1 = s_ci2[0][tid].y;
@@ -600,17 +646,25 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
     // the buffer fields of pair p + 1 load while pair p is computed (those
     // of pair 0 while the channel part runs)
     V nb0, nb1, nb2, nb3, nb4, nb5;
-    {
+    if (subs) {
+      const uint32_t g0 = SPLIT ? pair * S + g : g;
       const V* b2 = reinterpret_cast<const V*>(L.catf);
-      nb0 = b2[g];
-      nb1 = reinterpret_cast<const V*>(L.cats)[g];
-      nb2 = reinterpret_cast<const V*>(L.cacal)[g];
-      nb3 = reinterpret_cast<const V*>(L.casr)[g];
-      nb4 = reinterpret_cast<const V*>(L.camyo)[g];
-      nb5 = reinterpret_cast<const V*>(L.mgmyo)[g];
+      nb0 = b2[g0];
+      nb1 = reinterpret_cast<const V*>(L.cats)[g0];
+      nb2 = reinterpret_cast<const V*>(L.cacal)[g0];
+      nb3 = reinterpret_cast<const V*>(L.casr)[g0];
+      nb4 = reinterpret_cast<const V*>(L.camyo)[g0];
+      nb5 = reinterpret_cast<const V*>(L.mgmyo)[g0];
     }
 
+    const bool line = OUT && out_step && a.out_ls && y == sh.line_y && z == sh.line_z;
+    double* line_row = nullptr;
+    if (line) line_row = a.out_ls + ((size_t)sh.ls_off + (size_t)sh.slot * lx + x) * RH_LINESCAN_COLS;
+    double* cadist_row = nullptr;
+    if (OUT && cadist_step)  // this CRU's slot
+      cadist_row = a.out_cd + sh.cd_off + sh.cd_slot * (2 + 6 * (long long)sh.n) + 2 + 6 * (long long)q;
 
+    if (channel) {
     // ---- CRU state of the stochastic part ----
     R cjsrb = kSS ? s_sc[2][tid] : L.cjsrb[g], ancx = kSS ? s_sc[3][tid] : L.ancx[g];
     const uint32_t ryr = kSS ? s_ryr[tid] : L.ryr[g];
@@ -782,6 +836,72 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
       a.diag[(int64_t)D_XICAT * S + g] = (double)(icat1 + bcgcur * R(VS / VP));
     }
     tstat = status;
+    p_cs = csn;
+    p_xicat = icat1 + bcgcur * R(VS / VP);  // xicat (:1271)
+    p_xinaca = xinaca;
+    if (OUT && out_step) {
+      o[O_CP - P_STEP_END] = cp;
+      o[O_CJSR - P_STEP_END] = cjsr;
+      o[O_CJSRB - P_STEP_END] = cjsrb;
+      o[O_PO - P_STEP_END] = po;
+      o[O_NCB - P_STEP_END] = ncb;
+      o[O_NCXFWD - P_STEP_END] = xinaca < R(0) ? xinaca : R(0);
+      o[O_XIRE - P_STEP_END] = xire;
+      o[O_ANCX - P_STEP_END] = ancx;
+      o[O_CASAR - P_STEP_END] = casar;
+      o[O_CASARH - P_STEP_END] = casarh;
+      o[O_CASARJ - P_STEP_END] = casarj;
+      o[O_CASARHJ - P_STEP_END] = casarhj;
+      o[O_NOU - P_STEP_END] = nou;
+      o[O_NOB - P_STEP_END] = nob;
+      o[O_NCU - P_STEP_END] = ncu;
+      {
+        int tn[7] = {0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+        for (int ll = 0; ll < 8; ++ll) {
+          int st = ((ll < 4 ? lccw.x : lccw.y) >> ((ll & 3) * 8)) & 0xff;
+          if (st < 16) {
+            tn[0] += st & 1;
+            tn[1] += (st >> 1) & 1;
+            tn[2] += (st >> 2) & 1;
+            tn[3] += (st >> 3) & 1;
+            tn[4] += ((st >> 2) & 3) == 1;
+            tn[5] += st <= 1;
+            tn[6] += st == 0;
+          }
+        }
+#pragma unroll
+        for (int kk = 0; kk < 7; ++kk) o[O_TN1 - P_STEP_END + kk] = tn[kk];
+      }
+      o[O_SPARK - P_STEP_END] = nspark;
+      if (cadist_step) {  // cadist row (:1009), post-step values; ci below
+        double* r = cadist_row;
+        r[1] = (double)csn;
+        r[2] = (double)cp;
+        r[3] = (double)cjsr;
+        r[4] = (double)xinaca;  // scaled on the host as the reference prints it
+        r[5] = (double)xire;
+      }
+      if (line) {  // linescan row (:967-989), post-step values; the sub-voxel ones below
+        double* r = line_row;
+        r[0] = sh.t;
+        r[1] = (double)(x + 1);
+        r[3] = nob;
+        r[4] = nou;
+        r[5] = ncb;
+        r[6] = ncu;
+        r[7] = nl;
+        r[8] = (double)csn;
+        r[9] = (double)cp;
+        r[10] = (double)casar;
+        r[11] = (double)casarh;
+        r[18] = (double)xire;
+        r[19] = (double)cjsr;
+        r[20] = (double)ancx;
+        r[21] = (double)xinaca;
+      }
+    }
+    }  // channel
 
     // the channel part above reads no halo; the sub-voxel part below needs
     // this thread's halo copies
@@ -824,12 +944,12 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
     R sum_camyo = R(0), sum_cacal = R(0), sum_up = R(0), sum_lk = R(0);
     bool ci_high = false;
 #pragma unroll 1
-    for (int p = 0; p < 4; ++p) {
+    for (int p = SPLIT ? pair : 0; subs && p < (SPLIT ? pair + 1 : 4); ++p) {
       const int by = p & 1, bx = p >> 1;
       const uint32_t gp = p * S + g;
       const V c = s_ci2[p][tid], n = s_cn2[p][tid];
       V catf = nb0, cats = nb1, cacal = nb2, casr = nb3, camyo = nb4, mgmyo = nb5;
-      if (p < 3) {
+      if (!SPLIT && p < 3) {
         const uint32_t gq = gp + S;
         nb0 = catf2[gq], nb1 = cats2[gq], nb2 = cacal2[gq], nb3 = casr2[gq], nb4 = camyo2[gq];
         nb5 = mgmyo2[gq];
@@ -1049,94 +1169,47 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
         sum_up += up.x + up.y;
         sum_lk += lk.x + lk.y;
         ci_high |= (cinew.x > R(1000)) || (cinew.y > R(1000));
-      }
-    }
-
-    p_cs = csn;
-    p_xicat = icat1 + bcgcur * R(VS / VP);  // xicat (:1271)
-    p_xinaca = xinaca;
-
-    if (OUT && out_step) {
-      o[O_CP - P_STEP_END] = cp;
-      o[O_CJSR - P_STEP_END] = cjsr;
-      o[O_CJSRB - P_STEP_END] = cjsrb;
-      o[O_CNSR - P_STEP_END] = sum_cn;
-      o[O_CI - P_STEP_END] = sum_ci;
-      o[O_PO - P_STEP_END] = po;
-      o[O_NCB - P_STEP_END] = ncb;
-      o[O_NCXFWD - P_STEP_END] = xinaca < R(0) ? xinaca : R(0);
-      o[O_CATF - P_STEP_END] = sum_catf;
-      o[O_CATS - P_STEP_END] = sum_cats;
-      o[O_CASR - P_STEP_END] = sum_casr;
-      o[O_CAMYO - P_STEP_END] = sum_camyo;
-      o[O_CACAL - P_STEP_END] = sum_cacal;
-      o[O_LEAK - P_STEP_END] = sum_lk;
-      o[O_UP - P_STEP_END] = sum_up;
-      o[O_XIRE - P_STEP_END] = xire;
-      o[O_ANCX - P_STEP_END] = ancx;
-      o[O_CASAR - P_STEP_END] = casar;
-      o[O_CASARH - P_STEP_END] = casarh;
-      o[O_CASARJ - P_STEP_END] = casarj;
-      o[O_CASARHJ - P_STEP_END] = casarhj;
-      o[O_NOU - P_STEP_END] = nou;
-      o[O_NOB - P_STEP_END] = nob;
-      o[O_NCU - P_STEP_END] = ncu;
-      {
-        int tn[7] = {0, 0, 0, 0, 0, 0, 0};
-#pragma unroll
-        for (int ll = 0; ll < 8; ++ll) {
-          int st = ((ll < 4 ? lccw.x : lccw.y) >> ((ll & 3) * 8)) & 0xff;
-          if (st < 16) {
-            tn[0] += st & 1;
-            tn[1] += (st >> 1) & 1;
-            tn[2] += (st >> 2) & 1;
-            tn[3] += (st >> 3) & 1;
-            tn[4] += ((st >> 2) & 3) == 1;
-            tn[5] += st <= 1;
-            tn[6] += st == 0;
-          }
+        if (p == 0 && cadist_step) cadist_row[0] = (double)cinew.x;
+        if (p == 0 && line) {
+          line_row[2] = (double)cinew.x;
+          line_row[12] = (double)camyo.x;
+          line_row[13] = (double)mgmyo.x;
+          line_row[14] = (double)casr.x;
+          line_row[15] = (double)cacal.x;
+          line_row[16] = (double)cats.x;
+          line_row[17] = (double)catf.x;
         }
-#pragma unroll
-        for (int kk = 0; kk < 7; ++kk) o[O_TN1 - P_STEP_END + kk] = tn[kk];
-      }
-      o[O_SPARK - P_STEP_END] = nspark;
-      o[O_CIHIGH - P_STEP_END] = ci_high ? R(1) : R(0);
-      if (cadist_step) {  // cadist row (:1009), post-step values in this CRU's slot
-        double* r = a.out_cd + sh.cd_off + sh.cd_slot * (2 + 6 * (long long)sh.n) + 2 + 6 * (long long)q;
-        r[0] = (double)cinext2[g].x;
-        r[1] = (double)csn;
-        r[2] = (double)cp;
-        r[3] = (double)cjsr;
-        r[4] = (double)xinaca;  // scaled on the host as the reference prints it
-        r[5] = (double)xire;
-      }
-      if (a.out_ls && y == sh.line_y && z == sh.line_z) {  // linescan row (:967-989), post-step values
-        const uint32_t g0 = g;
-        double* r = a.out_ls + ((size_t)sh.ls_off + (size_t)sh.slot * lx + x) * RH_LINESCAN_COLS;
-        r[0] = sh.t;
-        r[1] = (double)(x + 1);
-        r[2] = (double)cinext2[g0].x;
-        r[3] = nob;
-        r[4] = nou;
-        r[5] = ncb;
-        r[6] = ncu;
-        r[7] = nl;
-        r[8] = (double)csn;
-        r[9] = (double)cp;
-        r[10] = (double)casar;
-        r[11] = (double)casarh;
-        r[12] = (double)L.camyo[2 * g0];
-        r[13] = (double)L.mgmyo[2 * g0];
-        r[14] = (double)L.casr[2 * g0];
-        r[15] = (double)L.cacal[2 * g0];
-        r[16] = (double)L.cats[2 * g0];
-        r[17] = (double)L.catf[2 * g0];
-        r[18] = (double)xire;
-        r[19] = (double)cjsr;
-        r[20] = (double)ancx;
-        r[21] = (double)xinaca;
       }
     }
+
+    if (OUT && out_step && subs) {
+      const R sums[kPairSums] = {sum_cn,   sum_ci,    sum_catf, sum_cats, sum_casr,
+                                 sum_camyo, sum_cacal, sum_lk,  sum_up,   ci_high ? R(1) : R(0)};
+      if constexpr (SPLIT) {
+#pragma unroll
+        for (int i = 0; i < kPairSums; ++i) s_sum[pair][i][tid] = sums[i];
+      } else {
+#pragma unroll
+        for (int i = 0; i < kPairSums; ++i) o[kPairSumOf[i] - P_STEP_END] = sums[i];
+      }
+    }
+  }
+
+  if constexpr (SPLIT) {
+    if (OUT && out_step) {
+      __syncthreads();
+      if (channel && valid) {  // the pairs' sums, in their order
+#pragma unroll
+        for (int i = 0; i < kPairSums; ++i) {
+          R t = s_sum[0][i][tid];
+          const R t1 = s_sum[1][i][tid], t2 = s_sum[2][i][tid], t3 = s_sum[3][i][tid];
+          if (i == kPairSums - 1) t = fmax(fmax(t, t1), fmax(t2, t3));
+          else t = t + t1 + t2 + t3;
+          o[kPairSumOf[i] - P_STEP_END] = t;
+        }
+      }
+    }
+    if (!channel) return true;
   }
 
   // every thread waits for the halo rows, so no bulk copy is still writing
