@@ -1054,21 +1054,16 @@ __device__ __forceinline__ bool tile_update(const StepArgs<R>& a, int ti, TileHe
         cix_ex = ci_ex;
         cnx_ex = cn_ex;
       }
-      // sums of the pair's differences along z: the halves' own difference
-      // enters both with opposite signs, which saves an FP64 subtraction
-      V cnz, ciz;
+      V coupn, coupi;
       if constexpr (sizeof(R) == 8) {
-        const R dn = n.y - n.x, dc = c.y - c.x;
-        cnz = v2(dn + (cnS.x - n.x), (cnN.y - n.y) - dn);
-        ciz = v2(dc + (ciS.x - c.x), (ciN.y - c.y) - dc);
+        coupn = stencil_pair(n, cnS.x, cnN.y, cny_in, cny_ex, cnx_in, cnx_ex, kt_n.x, kl_n.x);
+        coupi = stencil_pair(c, ciS.x, ciN.y, ciy_in, ciy_ex, cix_in, cix_ex, kt_i.x, kl_i.x);
       } else {
-        cnz = vadd(vsub(cnN, n), vsub(cnS, n));
-        ciz = vadd(vsub(ciN, c), vsub(ciS, c));
+        coupn = vfma(vadd(vadd(vadd(vsub(cnN, n), vsub(cnS, n)), vsub(cny_in, n)), vsub(cny_ex, n)),
+                     kt_n, vmul(vadd(vsub(cnx_in, n), vsub(cnx_ex, n)), kl_n));
+        coupi = vfma(vadd(vadd(vadd(vsub(ciN, c), vsub(ciS, c)), vsub(ciy_in, c)), vsub(ciy_ex, c)),
+                     kt_i, vmul(vadd(vsub(cix_in, c), vsub(cix_ex, c)), kl_i));
       }
-      const V coupn = vfma(vadd(vadd(cnz, vsub(cny_in, n)), vsub(cny_ex, n)), kt_n,
-                           vmul(vadd(vsub(cnx_in, n), vsub(cnx_ex, n)), kl_n));
-      const V coupi = vfma(vadd(vadd(ciz, vsub(ciy_in, c)), vsub(ciy_ex, c)), kt_i,
-                           vmul(vadd(vsub(cix_in, c), vsub(cix_ex, c)), kl_i));
       // SERCA and leak (subroutine_cuda.c:128-146)
       V up, lk;
       {

@@ -78,3 +78,36 @@ def test_fp64_channel_draws_are_those_of_the_fp64_comparisons(seed, v, params):
         got = sim.get_state(0)
     bad = count_mismatch(got, o.get_state())
     assert not bad.any(), np.flatnonzero(bad)[:10]
+
+
+@pytest.mark.parametrize("kind", ["smooth", "wide", "with_zeros"])
+def test_fp64_stencil_sums_match_oracle(kind):
+    """One lattice step from sub-voxel fields that are nearly constant (the
+    sums cancel), spread over five decades (mantissas shifted out) or zero in
+    places (the FP64 form): ci and cnsr within a few units in the last place of
+    the largest value around."""
+    from oracle import oracle as O
+
+    p = cell_params(nx=11, ny=9, nz=6, lqt=0, tapsi=1)  # no SERCA
+    o = O.Oracle(p)
+    st, m = o.get_state(), o.get_membrane()
+    rng = np.random.default_rng(8)
+    for f, level in (("ci", 0.1), ("cnsr", 500.0)):
+        n = st[f].size
+        if kind == "smooth":
+            st[f][...] = level * (1 + 1e-6 * rng.standard_normal(n))
+        else:
+            st[f][...] = level * np.exp(rng.uniform(-6, 6, n))
+        if kind == "with_zeros":
+            st[f][rng.random(n) < 0.2] = 0.0
+    o.set_state(st)
+    o.set_membrane(m)
+    o.lattice_step()
+    ref = o.get_state()
+    with Simulator(p, precision="fp64") as sim:
+        sim.set_state(0, st)
+        sim.set_membrane(0, m)
+        sim.lattice_step()
+        got = sim.get_state(0)
+    for f in ("ci", "cnsr"):
+        assert np.max(np.abs(got[f] - ref[f])) <= 1e-14 * max(st[f].max(), ref[f].max()), f
