@@ -344,21 +344,24 @@ __device__ __forceinline__ R buffer_rate(R kon, R koff, R total, R bound, R c, R
   return on * (total - bound) - koff * bound;
 }
 
-// ---- the FP64 lattice's stencil sums in integers ----
+// ---- the FP64 lattice's sums in integers ----
 //
 // A sub-voxel's diffusion needs the sum of its four transverse neighbours less
 // four times itself and of its two longitudinal ones less twice itself: 23 FP64
-// instructions for a z-pair of one field, of 4.  The mantissas are instead
-// aligned to the largest exponent among the pair's twelve values and summed as
-// 64-bit integers, then rounded once: exact where the values lie within a
-// factor of 32 of the largest, else an error of at most 2^-54 of the largest
-// value, where the FP64 differences round at 2^-53 of it.  The FP64 kernel is
-// bound by the FP64 pipe (19 cycles of an SM per warp instruction) and issues
-// in an eighth of its cycles; the integer instructions fit in the rest.  100
-// steps of the 64-cell FP64 ensemble: 92.6 ms with the FP64 sums, 80.8 so.
+// instructions for a z-pair of one field, of 4.  The values' mantissas are
+// instead aligned to the largest exponent among them and summed as 64-bit
+// integers, then rounded once: exact where the values lie within a factor of 32
+// of the largest, else with an error of at most 2^-54 of the largest, where the
+// FP64 differences round at 2^-53 of it (mean error relative to the largest
+// value 4.4e-17 against 6.9e-17).  The FP64 kernel is bound by the FP64 pipe
+// (19 cycles of an SM per warp instruction) and issues in an eighth of its
+// cycles; the integer instructions fit in the rest.  100 steps of the 64-cell
+// FP64 ensemble: 92.6 ms with the FP64 sums, 80.9 so.  The seven rates of a
+// sub-voxel's balance and the buffers' free sites summed this way as well were
+// slower (83.5 ms).
 
-// Mantissa of a positive normal v, aligned to the biased exponent e >= v's,
-// with five bits below the largest value's last.
+// Mantissa of v >= 0 aligned to the biased exponent e >= v's, with five bits
+// below the largest value's last (0 and subnormals are shifted out).
 __device__ __forceinline__ int64_t aligned_mantissa(double v, int e) {
   const int hi = __double2hiint(v);
   const uint64_t m = ((uint64_t)(uint32_t)((hi & 0xfffff) | 0x100000) << 32) |
@@ -380,39 +383,36 @@ __device__ __forceinline__ double from_aligned(int64_t t, int e) {
 
 // kt (transverse sum) + kl (longitudinal sum) of a z-pair c: its outer
 // neighbours along z (zs of the lower half, zn of the upper), and the inner
-// and outer neighbour pairs along y and x.
+// and outer neighbour pairs along y and x.  Each half is aligned to its own
+// largest value.
 __device__ __forceinline__ double2 stencil_pair(double2 c, double zs, double zn, double2 yi,
                                                 double2 ye, double2 xi, double2 xe, double kt,
                                                 double kl) {
-  const double v[12] = {c.x, c.y, zs, zn, yi.x, yi.y, ye.x, ye.y, xi.x, xi.y, xe.x, xe.y};
-  uint32_t a[12], b[12];  // largest and smallest high word, as trees
-#pragma unroll
-  for (int i = 0; i < 12; ++i) a[i] = b[i] = (uint32_t)__double2hiint(v[i]);
-#pragma unroll
-  for (int k = 6; k > 1; k = (k + 1) / 2)  // 12, 6, 3, 2
-#pragma unroll
-    for (int i = 0; i < k; ++i) {
-      const int j = i + k < (k == 2 ? 3 : 2 * k) ? i + k : i;
-      a[i] = max(a[i], a[j]);
-      b[i] = min(b[i], b[j]);
-    }
-  const uint32_t hi = max(a[0], a[1]), lo = min(b[0], b[1]);
-  if (hi >= 0x7ff00000u || lo < 0x10000000u) {  // negative, zero, tiny, infinite or NaN among them
+  auto word = [](double x) { return (uint32_t)__double2hiint(x); };
+  const uint32_t own = max(word(c.x), word(c.y));
+  const uint32_t hx = max(max(max(word(zs), word(yi.x)), max(word(ye.x), word(xi.x))),
+                          max(own, word(xe.x)));
+  const uint32_t hy = max(max(max(word(zn), word(yi.y)), max(word(ye.y), word(xi.y))),
+                          max(own, word(xe.y)));
+  if (max(hx, hy) >= 0x7ff00000u || min(hx, hy) < 0x10000000u) {
+    // negative, infinite or NaN among them, or all tiny
     const double d = c.y - c.x;
     const double tx = (d + (zs - c.x)) + (yi.x - c.x) + (ye.x - c.x);
     const double ty = ((zn - c.y) - d) + (yi.y - c.y) + (ye.y - c.y);
     return make_double2(fma(tx, kt, __dmul_rn((xi.x - c.x) + (xe.x - c.x), kl)),
                         fma(ty, kt, __dmul_rn((xi.y - c.y) + (xe.y - c.y), kl)));
   }
-  const int e = (int)(hi >> 20);
-  int64_t m[12];
-#pragma unroll
-  for (int i = 0; i < 12; ++i) m[i] = aligned_mantissa(v[i], e);
-  const double tx = from_aligned(m[1] + m[2] + m[4] + m[6] - 4 * m[0], e);
-  const double ty = from_aligned(m[0] + m[3] + m[5] + m[7] - 4 * m[1], e);
-  const double lx = from_aligned(m[8] + m[10] - 2 * m[0], e);
-  const double ly = from_aligned(m[9] + m[11] - 2 * m[1], e);
-  return make_double2(fma(tx, kt, __dmul_rn(lx, kl)), fma(ty, kt, __dmul_rn(ly, kl)));
+  auto half = [&](uint32_t h, double c0, double c1, double z, double y0, double y1, double x0,
+                  double x1) {
+    const int e = (int)(h >> 20);
+    const int64_t m = aligned_mantissa(c0, e);
+    const int64_t t = (aligned_mantissa(c1, e) + aligned_mantissa(z, e)) +
+                      (aligned_mantissa(y0, e) + aligned_mantissa(y1, e)) - 4 * m;
+    const int64_t l = aligned_mantissa(x0, e) + aligned_mantissa(x1, e) - 2 * m;
+    return fma(from_aligned(t, e), kt, __dmul_rn(from_aligned(l, e), kl));
+  };
+  return make_double2(half(hx, c.x, c.y, zs, yi.x, ye.x, xi.x, xe.x),
+                      half(hy, c.y, c.x, zn, yi.y, ye.y, xi.y, xe.y));
 }
 
 // ---- CSQN (subroutine_cuda.c:161-195) ----
