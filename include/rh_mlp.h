@@ -62,7 +62,8 @@ int rh_mlp_last_error(const rh_mlp* m, char* buf, size_t n);
  *
  * The intermediate values live in the kernel's shared memory: the library
  * keeps no array for them, and calls on different streams or threads are
- * independent.  n above RH_MLP_NOALLOC_MAX_BATCH is rejected with RH_ERR_ARG
+ * independent.  The first call on a device sets the kernel up (once, by the
+ * runtime); make it before any stream capture.  n above RH_MLP_NOALLOC_MAX_BATCH is rejected with RH_ERR_ARG
  * and a message in err (err may be NULL). */
 /* Check of the library's GEMM kernels (testing aid; synchronous, default
  * stream): C[M x N] (FP32, row-major, leading dimension ldc) = sum over k of

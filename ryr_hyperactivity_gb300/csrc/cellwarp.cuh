@@ -8,8 +8,8 @@
 // lane; here every group of mutually independent transcendentals and
 // divisions is evaluated in one SIMT call, one operand set per lane, through
 // a 32-slot shared-memory exchange.  Each operation keeps its operands and
-// its order, so the results are bit-identical to the serial versions; only
-// the lane that computes each value changes.  The reference's two powers,
+// its order; only the lane that computes each value changes.  (cellwide.cuh
+// spreads the same work over four warps.)  The reference's two powers,
 // pow(0.28/csubt, 3) and pow(12/xnai, 1), are a product and the quotient
 // itself in both versions (the CPU oracle keeps pow; the results differ in
 // the last bits).

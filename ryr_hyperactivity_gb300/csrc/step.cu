@@ -12,7 +12,8 @@
 //      fixed point (fixedsum.cuh) and adds them to the cell's accumulators
 //      with integer atomics; at output steps it also stores the ~30
 //      statistics of :839-929 as one FP64 partial row per warp;
-//   2. cell_kernel, next on the same stream: one warp per cell reads the
+//   2. cell_kernel (cell_wide_kernel for small simulations), next on the
+//      same stream: one warp (four) per cell reads the
 //      sums (and sums the output partials in a fixed order), runs the
 //      membrane model and V update (:430-739, the reference's host loop),
 //      writes the output record at output steps, and prepares the
