@@ -342,7 +342,9 @@ typedef struct {
                            asynchronous copies issued by one warp (completion
                            on mbarriers); 2 = the tile's ci/cnsr pair planes and
                            its eight real planes arrive as 2-D tensor tiles
-                           (cp.async.bulk.tensor, one thread), the rest as in 0 */
+                           (cp.async.bulk.tensor, one thread), the rest as in 0.
+                           While no shape was asked for, large ensembles run 2,
+                           with the same results */
 } rh_launch_shape;
 
 int rh_get_launch_shape(const rh_sim* sim, rh_launch_shape* shape);

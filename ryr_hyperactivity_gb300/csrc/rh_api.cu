@@ -358,6 +358,20 @@ bool split_tiles(const rh_sim* s) {
   return active_set(s) == kNarrowSet && (s->ngroups > 1 || tiles <= wave || tiles >= 2 * wave);
 }
 
+// Staging of the FP32 lattice launches: the launch shape's, or while none was
+// asked for tensor copies from three waves of tiles on.  They take the own
+// planes' copies off the threads, which pays once CTAs follow one another
+// (per-thread against tensor copies, 100 steps: 512 cells 49.67 and 49.36 ms,
+// 256 cells 24.29 and 24.19, 60 cells 5.88 and 5.85), while in the first wave
+// their barrier initialisation and waits cost more (200 cells of 432 CRUs
+// 2.83 and 2.85 ms, 50 cells 1.73 and 1.75).  The same results.
+int lattice_staging(const rh_sim* s) {
+  if (split_tiles(s)) return 3;
+  const int64_t wave = (int64_t)min_blocks_for<float, kDefaultTile>() * s->sm_count;
+  const bool many = active_set(s) == s->ts && s->sets[s->ts].ntiles >= 3 * wave;
+  return !s->shape_given && s->maps_ok && many ? 2 : s->staging;
+}
+
 // One group's step: the tiles of cells [group_cell[g], group_cell[g+1]),
 // then the whole-cell update of those cells.
 cudaError_t launch_group(rh_sim* s, int g, bool out, bool lattice_only, cudaStream_t st) {
@@ -371,7 +385,7 @@ cudaError_t launch_group(rh_sim* s, int g, bool out, bool lattice_only, cudaStre
     a.tiles += tb;
     a.tile_base = tb;
     if ((e = launch_step<float>(a, te - tb, out, s->group_opt[g], t.tile,
-                                split_tiles(s) ? 3 : s->staging,
+                                lattice_staging(s),
                                 &s->maps[s->ts], st)) != cudaSuccess)
       return e;
     return launch_cells<float>(a, c0, c1 - c0, out, t.tile, wide_cells(s), st);

@@ -1,6 +1,7 @@
 """The narrow tiles the library uses for small lattices by itself (32 CRUs by
-five warps or one) give the state and records of the default tiles, in both
-precisions and with the build options' kernel variant."""
+five warps or one), and the staging it chooses for large ones, give the state
+and records of the default launch shape, in both precisions and with the build
+options' kernel variant."""
 import numpy as np
 import pytest
 
@@ -24,6 +25,7 @@ def _run(cells, precision, **opts):
     ([(10, 6, 3)], [{}]),                         # exactly one tile
     ([(35, 9, 4)], [{}]),                         # a row longer than a tile, one CRU over
     ([(60, 24, 17)], [{}]),                       # too many tiles for five warps each
+    ([(100, 60, 30), (99, 61, 30)], [{}, {}]),    # three waves of default tiles: tensor copies
     ([(12, 7, 5), (41, 8, 6), (5, 4, 13)], [{}, dict(perm=1), dict(slowncx=1, ncx_form="oldncx")]),
 ])
 def test_narrow_tiles_equal_default_tiles(precision, extents, options):
