@@ -321,20 +321,49 @@ __device__ inline void wholecell_columns_warp(double* w, const double* o, const 
 }
 
 // Output-step partials of one cell, one row per warp of each of its tiles:
-// lane q sums statistic q over the rows in order into o[q]; the ci > 1000
-// flag (the last one) is a maximum.  A warp's FP64 additions cost the same
-// with one lane or 32, so a statistic per lane beats a row per lane with a
-// reduction for each of 33 statistics (441 rows: 441 against 630).
+// lane q sums statistic q over the rows into o[q]; the ci > 1000 flag (the
+// last one) is a maximum.  Row r joins partial sum r % 32 and the 32 partial
+// sums are added pairwise (16 apart, then 8, 4, 2, 1): one sum over 441 rows
+// would be off by 14 times as much, over 5,100 by 25 times.  A warp's FP64
+// additions cost the same with one lane or 32, so a statistic per lane beats a
+// partial sum per lane with a reduction for each of the 33 statistics (441
+// rows: 480 additions against 630).  Eight groups of four partial sums, four
+// loads in flight each, taken in the order in which the pairs of the tree
+// close, so that three pending sums are all that is kept.
 __device__ inline void output_sums_warp(const double* partials, int nrows, double* o, int lane) {
   static_assert(O_CIHIGH - P_STEP_END == NOUT - 1 && NOUT - 1 == 32, "one statistic per lane");
-  double s = 0.0;
+  const double* p = partials + P_STEP_END + lane;
+  double pending[3] = {0.0, 0.0, 0.0}, t = 0.0;
+#pragma unroll 1
+  for (int i = 0; i < 8; ++i) {
+    const int j = (int)(__brev((unsigned)i) >> 29);  // partial sums j, j + 8, j + 16, j + 24
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+    for (int r = j; r < nrows; r += 32) {
+      double v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        v[q] = r + 8 * q < nrows ? __ldcg(p + (size_t)(r + 8 * q) * P_COUNT) : 0.0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) s[q] += v[q];
+    }
+    t = (s[0] + s[2]) + (s[1] + s[3]);
+    bool open = true;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      if (open && (i >> b & 1)) {
+        t = pending[b] + t;
+      } else if (open) {
+        pending[b] = t;
+        open = false;
+      }
+    }
+  }
   bool high = false;
-#pragma unroll 4
-  for (int r = 0; r < nrows; ++r) s += __ldcg(partials + (size_t)r * P_COUNT + P_STEP_END + lane);
   for (int r = lane; r < nrows; r += 32)
     high |= __ldcg(partials + (size_t)r * P_COUNT + O_CIHIGH) > 0.0;
   high = __any_sync(0xffffffffu, high);
-  o[lane] = s;
+  o[lane] = t;
   if (lane == 0) o[NOUT - 1] = high ? 1.0 : 0.0;
   __syncwarp();
 }
