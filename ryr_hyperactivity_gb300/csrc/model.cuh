@@ -636,6 +636,7 @@ __device__ __forceinline__ bool ryr_draws_estimated(rh_stream* rng, const StepCo
   const float q = __fdividef(5000.0f, narrow(cjsr, ok));
   const float a = __fdividef(narrow(k.ku, ok), narrow(cp, ok));
   const float common = __fdividef(1.0f, (1.0f + q * q) * (1.0f + a * a));
+  ok = ok && common >= 0.0f;  // 0/0 among the quotients: the minimum below would hide the NaN
   const float step = fminf(dt, 1.0f);  // the rates of 1 per ms, capped
   const float pku = fminf(float(4.5 * 1.5) * narrow(k.ku2, ok) * common * dt, 1.0f);
   const float pkb0 = float(4.5 * 1.5 / 36.) * narrow(k.kb, ok) * common;

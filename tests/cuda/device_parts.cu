@@ -29,6 +29,33 @@ __global__ void sums_kernel(const double* rows, int n, double* o) {
   output_sums_warp(rows, n, o, (int)threadIdx.x);
 }
 
+// RyR transition counts of CRU i by the FP32 estimates and by the FP64
+// comparisons; est[i]: the estimates decided them all.
+__global__ void draws_kernel(int n, const double* cp, const double* cjsr, const double* mono,
+                             const double* ku, const double* ku2, const double* kb, double dt,
+                             const int* counts, uint32_t* est, uint32_t* e, uint32_t* x) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  StepCoef<double> k{};
+  k.ku = ku[i];
+  k.ku2 = ku2[i];
+  k.kb = kb[i];
+  k.dt = dt;
+  k.rdt = 1.0 / dt;
+  rh_stream a, b;
+  rh_stream_init(&a, 7u, 3u, (uint32_t)i, 5u);
+  b = a;
+  const int* c = counts + 4 * i;
+  uint32_t status = 0;
+  est[i] = ryr_draws_estimated(&a, k, cp[i], cjsr[i], mono[i], c[0], c[1], c[2], c[3], e[2 * i],
+                               e[2 * i + 1])
+               ? 1u + a.draw
+               : 0u;
+  ryr_draws<double, 1>(&b, k, cp[i], cjsr[i], mono[i], c[0], c[1], c[2], c[3], x[2 * i],
+                       x[2 * i + 1], &status);
+  if (est[i] && est[i] != 1u + b.draw) est[i] = 0xffffffffu;  // another number of draws taken
+}
+
 }  // namespace
 
 extern "C" {
@@ -41,6 +68,19 @@ int part_output_sums(const double* rows, int n, double* o) {
   Dev<double> r(rows, (size_t)n * P_COUNT), d(nullptr, NOUT);
   sums_kernel<<<1, 32>>>(r.p, n, d.p);
   return d.get(o) ? NOUT : -1;
+}
+
+// `in`: cp, cjsr, mono, ku, ku2, kb (n each); `counts`: nou, ncu, nob, ncb of
+// each CRU; est, e[2n], x[2n] as in draws_kernel.
+int part_draws(int n, const double* in, double dt, const int* counts, uint32_t* est, uint32_t* e,
+               uint32_t* x) {
+  const size_t m = (size_t)n;
+  Dev<double> d(in, 6 * m);
+  Dev<int> c(counts, 4 * m);
+  Dev<uint32_t> de(nullptr, m), d0(nullptr, 2 * m), d1(nullptr, 2 * m);
+  draws_kernel<<<(n + 127) / 128, 128>>>(n, d.p, d.p + m, d.p + 2 * m, d.p + 3 * m, d.p + 4 * m,
+                                         d.p + 5 * m, dt, c.p, de.p, d0.p, d1.p);
+  return de.get(est) && d0.get(e) && d1.get(x) ? 0 : -1;
 }
 
 }  // extern "C"

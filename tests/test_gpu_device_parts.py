@@ -44,3 +44,34 @@ def test_output_sums_are_32_strided_sums_joined_by_a_tree(parts, rows):
         s[:off] = s[:off] + s[off:2 * off]
     np.testing.assert_array_equal(got[:-1], s[0, :-1])
     assert got[-1] == float(rows % 2)
+
+
+@pytest.mark.parametrize("dt", [0.025, 0.1, 2.0])
+def test_estimated_draws_are_the_fp64_ones_or_none(parts, dt):
+    """Wherever the FP32 estimates decide a CRU's RyR transitions, the counts
+    and the draws taken are those of the FP64 comparisons: over rates from
+    nothing to the cap, and inputs that are zero, tiny, huge, infinite or NaN,
+    alone and together (0/0 among the rates included)."""
+    rng = np.random.default_rng(int(1000 * dt))
+    n = 400_000
+    scale = [np.exp(rng.uniform(np.log(a), np.log(b), n)) for a, b in
+             [(1e-2, 300.0), (20.0, 1500.0), (1e-3, 1.0), (1e-1, 100.0), (1e-3, 10.0), (1e-3, 10.0)]]
+    odd = np.array([0.0, 5e-324, 1e-310, 1e-60, 1e-39, 1e39, 1e300, np.inf, np.nan, -1.0, -0.0])
+    v = np.stack(scale)
+    hit = rng.random(v.shape) < 0.15
+    hit[:, : n // 2] = False  # half of the CRUs are ordinary
+    v[hit] = rng.choice(odd, hit.sum())
+    both = slice(n - n // 8, n)  # closed RyRs on an empty dyad: ku / cp is 0/0
+    v[0, both], v[3, both] = 0.0, 0.0
+    counts = rng.multinomial(100, [0.02, 0.5, 0.03, 0.45], n).astype(np.int32)
+    few = slice(n // 4, n)
+    counts[few] = rng.integers(0, 2, (n - n // 4, 4))
+    est = np.zeros(n, np.uint32)
+    e, x = np.zeros((n, 2), np.uint32), np.zeros((n, 2), np.uint32)
+    v, counts = np.ascontiguousarray(v), np.ascontiguousarray(counts)
+    assert parts.part_draws(n, _p(v), C.c_double(dt), _p(counts), _p(est), _p(e), _p(x)) == 0
+    assert np.count_nonzero(est == 0xffffffff) == 0
+    bad = (est != 0) & (e != x).any(axis=1)
+    assert not bad.any(), (int(bad.sum()), v[:, bad][:, :5], counts[bad][:5])
+    if dt == 0.025:  # the model's step, no Gaussian draws: the estimates do decide
+        assert np.count_nonzero(est[: n // 2]) > 0.9 * (n // 2)
