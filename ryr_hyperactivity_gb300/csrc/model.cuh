@@ -394,8 +394,9 @@ __device__ __forceinline__ double2 stencil_pair(double2 c, double zs, double zn,
                           max(own, word(xe.x)));
   const uint32_t hy = max(max(max(word(zn), word(yi.y)), max(word(ye.y), word(xi.y))),
                           max(own, word(xe.y)));
-  if (max(hx, hy) >= 0x7ff00000u || min(hx, hy) < 0x10000000u) {
-    // negative, infinite or NaN among them, or all tiny
+  if (max(hx, hy) >= 0x7f000000u || min(hx, hy) < 0x10000000u) {
+    // negative, infinite, NaN or above 2^1009 (the sums can overflow, which
+    // from_aligned cannot express) among them, or all tiny
     const double d = c.y - c.x;
     const double tx = (d + (zs - c.x)) + (yi.x - c.x) + (ye.x - c.x);
     const double ty = ((zn - c.y) - d) + (yi.y - c.y) + (ye.y - c.y);

@@ -56,6 +56,17 @@ __global__ void draws_kernel(int n, const double* cp, const double* cjsr, const 
   if (est[i] && est[i] != 1u + b.draw) est[i] = 0xffffffffu;  // another number of draws taken
 }
 
+__global__ void stencil_kernel(int n, const double* v, double kt, double kl, double* o) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double* w = v + 12 * i;
+  const double2 r = stencil_pair(make_double2(w[0], w[1]), w[2], w[3], make_double2(w[4], w[5]),
+                                 make_double2(w[6], w[7]), make_double2(w[8], w[9]),
+                                 make_double2(w[10], w[11]), kt, kl);
+  o[2 * i] = r.x;
+  o[2 * i + 1] = r.y;
+}
+
 }  // namespace
 
 extern "C" {
@@ -81,6 +92,14 @@ int part_draws(int n, const double* in, double dt, const int* counts, uint32_t* 
   draws_kernel<<<(n + 127) / 128, 128>>>(n, d.p, d.p + m, d.p + 2 * m, d.p + 3 * m, d.p + 4 * m,
                                          d.p + 5 * m, dt, c.p, de.p, d0.p, d1.p);
   return de.get(est) && d0.get(e) && d1.get(x) ? 0 : -1;
+}
+
+// v: of each of n z-pairs its halves, outer z neighbours, inner and outer y
+// and x neighbour pairs (12 doubles); o: the pair's two sums
+int part_stencil(int n, const double* v, double kt, double kl, double* o) {
+  Dev<double> d(v, 12 * (size_t)n), r(nullptr, 2 * (size_t)n);
+  stencil_kernel<<<(n + 127) / 128, 128>>>(n, d.p, kt, kl, r.p);
+  return r.get(o) ? 0 : -1;
 }
 
 }  // extern "C"

@@ -75,3 +75,28 @@ def test_estimated_draws_are_the_fp64_ones_or_none(parts, dt):
     assert not bad.any(), (int(bad.sum()), v[:, bad][:, :5], counts[bad][:5])
     if dt == 0.025:  # the model's step, no Gaussian draws: the estimates do decide
         assert np.count_nonzero(est[: n // 2]) > 0.9 * (n // 2)
+
+
+@pytest.mark.parametrize("lo,hi", [(1e-300, 1e-100), (1e-3, 1e3), (1e290, 1.7e308)])
+def test_stencil_sums_equal_the_fp64_differences(parts, lo, hi):
+    """The integer sums against the same sums of FP64 differences: within the
+    rounding of both (8 differences of at most the largest value, a half unit
+    in the last place each), and overflowing where those overflow."""
+    rng = np.random.default_rng(2)
+    n, kt, kl = 100_000, 0.125, 0.03125
+    # neighbours within three decades of each other, at levels from lo to hi
+    level = np.exp(rng.uniform(np.log(lo), np.log(hi), (n, 1)))
+    v = np.minimum(level * np.exp(rng.uniform(-7, 0, (n, 12))), 1.79e308)
+    v[::7] = np.where(rng.random((len(v[::7]), 12)) < 0.5, v[::7], level[::7])
+    v = np.ascontiguousarray(v)
+    got = np.zeros((n, 2))
+    assert parts.part_stencil(n, _p(v), C.c_double(kt), C.c_double(kl), _p(got)) == 0
+    with np.errstate(over="ignore", invalid="ignore"):
+        for h in (0, 1):
+            c, z, far = v[:, h], v[:, 1 - h], v[:, 2 + h]
+            t = (((z - c) + (far - c)) + (v[:, 4 + h] - c)) + (v[:, 6 + h] - c)
+            want = t * kt + ((v[:, 8 + h] - c) + (v[:, 10 + h] - c)) * kl
+            inf = ~np.isfinite(want)
+            np.testing.assert_array_equal(got[inf, h], want[inf])
+            big = v.max(axis=1)
+            assert np.all(np.abs(got[~inf, h] - want[~inf]) <= 8 * 2.0**-53 * big[~inf])
