@@ -327,8 +327,8 @@ __device__ inline void wholecell_columns_warp(double* w, const double* o, const 
 // would be off by 14 times as much, over 5,100 by 25 times.  A warp's FP64
 // additions cost the same with one lane or 32, so a statistic per lane beats a
 // partial sum per lane with a reduction for each of the 33 statistics (441
-// rows: 480 additions against 630).  Eight groups of four partial sums, four
-// loads in flight each, taken in the order in which the pairs of the tree
+// rows: 480 additions against 630).  Eight groups of four partial sums, up
+// to 16 loads in flight, taken in the order in which the pairs of the tree
 // close, so that three pending sums are all that is kept.
 __device__ inline void output_sums_warp(const double* partials, int nrows, double* o, int lane) {
   static_assert(O_CIHIGH - P_STEP_END == NOUT - 1 && NOUT - 1 == 32, "one statistic per lane");
@@ -338,14 +338,15 @@ __device__ inline void output_sums_warp(const double* partials, int nrows, doubl
   for (int i = 0; i < 8; ++i) {
     const int j = (int)(__brev((unsigned)i) >> 29);  // partial sums j, j + 8, j + 16, j + 24
     double s[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 2
-    for (int r = j; r < nrows; r += 32) {
-      double v[4];
+#pragma unroll 1
+    for (int r = j; r < nrows; r += 128) {
+      double v[16];
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        v[q] = r + 8 * q < nrows ? __ldcg(p + (size_t)(r + 8 * q) * P_COUNT) : 0.0;
+      for (int q = 0; q < 16; ++q)
+        if (r + 8 * q < nrows) v[q] = __ldcg(p + (size_t)(r + 8 * q) * P_COUNT);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) s[q] += v[q];
+      for (int q = 0; q < 16; ++q)
+        if (r + 8 * q < nrows) s[q & 3] += v[q];
     }
     t = (s[0] + s[2]) + (s[1] + s[3]);
     bool open = true;
