@@ -67,6 +67,17 @@ __global__ void stencil_kernel(int n, const double* v, double kt, double kl, dou
   o[2 * i + 1] = r.y;
 }
 
+__global__ void serca_kernel(int n, const double* v, double sviup, double* o) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  serca_leak(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3], sviup, o[2 * i], o[2 * i + 1]);
+}
+
+__global__ void divide_kernel(int n, const double* a, const double* b, double* q) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) q[i] = div_refined(a[i], b[i]);
+}
+
 }  // namespace
 
 extern "C" {
@@ -100,6 +111,19 @@ int part_stencil(int n, const double* v, double kt, double kl, double* o) {
   Dev<double> d(v, 12 * (size_t)n), r(nullptr, 2 * (size_t)n);
   stencil_kernel<<<(n + 127) / 128, 128>>>(n, d.p, kt, kl, r.p);
   return r.get(o) ? 0 : -1;
+}
+
+// v: c, n, pa, pb of each of n sub-voxels; o: uptake and leak of each
+int part_serca_leak(int n, const double* v, double sviup, double* o) {
+  Dev<double> d(v, 4 * (size_t)n), r(nullptr, 2 * (size_t)n);
+  serca_kernel<<<(n + 127) / 128, 128>>>(n, d.p, sviup, r.p);
+  return r.get(o) ? 0 : -1;
+}
+
+int part_divide(int n, const double* a, const double* b, double* q) {
+  Dev<double> da(a, (size_t)n), db(b, (size_t)n), dq(nullptr, (size_t)n);
+  divide_kernel<<<(n + 127) / 128, 128>>>(n, da.p, db.p, dq.p);
+  return dq.get(q) ? 0 : -1;
 }
 
 }  // extern "C"

@@ -100,3 +100,59 @@ def test_stencil_sums_equal_the_fp64_differences(parts, lo, hi):
             np.testing.assert_array_equal(got[inf, h], want[inf])
             big = v.max(axis=1)
             assert np.all(np.abs(got[~inf, h] - want[~inf]) <= 8 * 2.0**-53 * big[~inf])
+
+
+@pytest.mark.parametrize("lo,hi", [(1e-3, 3e3), (1e-30, 1e30), (1e30, 1e160), (1e-320, 1e308)])
+def test_uptake_and_leak_equal_their_quotients(parts, lo, hi):
+    """SERCA uptake and leak, which share one reciprocal, against a division
+    each: within their roundings (at most six a side, a half unit in the last
+    place each), and infinite or NaN where those are."""
+    rng = np.random.default_rng(4)
+    m, sviup = 200_000, 0.91
+    v = np.exp(rng.uniform(np.log(lo), np.log(hi), (m, 4)))
+    if hi > 1e300:
+        odd = np.array([0.0, np.inf, np.nan, 5e-324, 1.79e308])
+        hit = rng.random((m, 2)) < 0.1
+        v[:, :2][hit] = rng.choice(odd, hit.sum())
+    with np.errstate(all="ignore"):
+        v[:, 2], v[:, 3] = (v[:, 0] / 0.123) ** 1.787, (v[:, 1] / 1700.0) ** 1.787
+        c, n, pa, pb = v.T
+        up = sviup * ((0.3 * (pa - pb)) / (1.0 + pa + pb))
+        lk = ((0.00001035 * (n - c)) * (n * n)) / (n * n + 500.0 * 500.0)
+    got = np.zeros((m, 2))
+    v = np.ascontiguousarray(v)
+    assert parts.part_serca_leak(m, _p(v), C.c_double(sviup), _p(got)) == 0
+    for g, want in ((got[:, 0], up), (got[:, 1], lk)):
+        np.testing.assert_array_equal(np.isnan(g), np.isnan(want))
+        ok = np.isfinite(want)
+        np.testing.assert_array_equal(g[np.isinf(want)], want[np.isinf(want)])
+        # below 1e-290 products of the numerators lose bits to underflow
+        tol = np.where(np.abs(want[ok]) > 1e-290, 12 * 2.0**-53 * np.abs(want[ok]), 1e-300)
+        assert np.all(np.abs(g[ok] - want[ok]) <= tol)
+
+
+@pytest.mark.parametrize("kind", ["model", "normal", "small_numerator", "any_bits", "special"])
+def test_refined_division_equals_the_rounded_quotient(parts, kind):
+    """div_refined against the correctly rounded quotient, bit for bit: the
+    model's magnitudes, all normal numbers, numerators whose residual is
+    subnormal, arbitrary bit patterns, and every pair of special values."""
+    rng = np.random.default_rng(6)
+    n = 4_000_000
+    special = np.array([0.0, 5e-324, 2.2e-308, 2.3e-308, 1e-290, 1e-20, 1.0, 3.0, 1e20, 1e290,
+                        1.7e308, np.inf, np.nan])
+    if kind == "special":
+        special = np.concatenate([special, -special])
+        a, b = (x.ravel() for x in np.meshgrid(special, special))
+    elif kind == "any_bits":
+        a, b = (rng.integers(0, 1 << 64, n, dtype=np.uint64).view(np.float64) for _ in range(2))
+    else:
+        def draw(lo, hi):
+            return np.ldexp(1.0 + rng.random(n), rng.integers(lo, hi, n)) * rng.choice([-1.0, 1.0], n)
+        e = {"model": (-40, 40), "normal": (-1022, 1024), "small_numerator": (-1022, -900)}[kind]
+        a, b = draw(*e), draw(*((-60, 60) if kind == "small_numerator" else e))
+    a, b, q = (np.ascontiguousarray(x, np.float64) for x in (a, b, np.zeros(len(a))))
+    assert parts.part_divide(len(a), _p(a), _p(b), _p(q)) == 0
+    with np.errstate(all="ignore"):
+        want = a / b
+    bad = (q.view(np.uint64) != want.view(np.uint64)) & ~(np.isnan(q) & np.isnan(want))
+    assert not bad.any(), (int(bad.sum()), a[bad][:5], b[bad][:5], q[bad][:5], want[bad][:5])
