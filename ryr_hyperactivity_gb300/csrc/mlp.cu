@@ -815,12 +815,11 @@ struct rh_mlp {
   float* P = nullptr;            // w, m, v, then the CTAs' gradients
   float *w = nullptr, *m = nullptr, *v = nullptr, *part = nullptr;
   unsigned char* img = nullptr;  // BF16 weights (kImgBytes)
-  // Host memory the kernels read and write directly (pinned, mapped): inputs
-  // of two chunks and targets of a batch (where the device cannot read the
-  // caller's own memory), outputs of two chunks or loss terms, gradients, the
-  // error flag.
+  // Host memory the kernels read and write directly (pinned, mapped): outputs
+  // of two chunks or loss terms, gradients, the error flag; and, made when first
+  // needed, copies of the caller's arrays (reachable(), below).
   unsigned char* host = nullptr;
-  float *h_x = nullptr, *h_t = nullptr, *h_out = nullptr, *h_g = nullptr;
+  float *h_out = nullptr, *h_g = nullptr, *copies = nullptr;
   int* h_err = nullptr;          // set by a pass whose wait gave up
   cudaEvent_t ev[2] = {nullptr, nullptr};
   bool direct = false;  // kernels can read pageable host memory (hardware page tables)
@@ -853,13 +852,25 @@ int check_wait(rh_mlp* m) {
 }
 
 // Where the kernels read `count` floats of the caller's `p`: in place, or
-// from a copy in `stage`.  In place is as fast or faster (a 65,536-point sweep
-// 95 against 130 us, gradients of 4,096 samples 58 against 64, a 256-sample
-// step 70 either way).
-const float* reachable(const rh_mlp* m, const float* p, size_t count, float* stage) {
-  if (m->direct) return p;
-  memcpy(stage, p, count * sizeof(float));
-  return stage;
+// from a pinned copy (kCopyX0, kCopyX1: inputs of a chunk; kCopyT: targets of
+// a batch) on a device that cannot read pageable memory, and of an array that
+// is not on a 4-byte boundary (numpy makes such arrays from the middle of a
+// buffer), which would fault a kernel's loads.  In place is as fast or faster
+// (a 65,536-point sweep 95 against 130 us, gradients of 4,096 samples 58
+// against 64, a 256-sample step 70 either way).
+enum CopySlot { kCopyX0, kCopyX1, kCopyT };
+int reachable(rh_mlp* m, const float* p, size_t count, CopySlot slot, const float** out) {
+  *out = p;
+  if (m->direct && reinterpret_cast<uintptr_t>(p) % alignof(float) == 0) return RH_OK;
+  const size_t nx = (size_t)m->chunk * RH_MLP_IN;
+  if (!m->copies)
+    MCK(cudaHostAlloc(reinterpret_cast<void**>(&m->copies),
+                      (2 * nx + (size_t)m->bmax * RH_MLP_OUT) * sizeof(float),
+                      cudaHostAllocMapped));
+  float* to = m->copies + (size_t)slot * nx;
+  memcpy(to, static_cast<const void*>(p), count * sizeof(float));
+  *out = to;
+  return RH_OK;
 }
 
 // One training pass: loss terms to h_out, each CTA's gradients to part.  A
@@ -874,8 +885,9 @@ int train_pass(rh_mlp* m, const float* x, const float* target, int n, int* npart
   RowsArgs a{};
   a.img = m->img;
   a.params = m->w;
-  a.x = reachable(m, x, (size_t)n * RH_MLP_IN, m->h_x);
-  a.target = reachable(m, target, (size_t)n * RH_MLP_OUT, m->h_t);
+  int r = reachable(m, x, (size_t)n * RH_MLP_IN, kCopyX0, &a.x);
+  if (r == RH_OK) r = reachable(m, target, (size_t)n * RH_MLP_OUT, kCopyT, &a.target);
+  if (r != RH_OK) return r;
   a.loss = m->h_out;
   a.part = m->part;
   a.n = n;
@@ -936,13 +948,11 @@ int rh_mlp_create(int32_t batch_max, int32_t device, rh_mlp** out) {
       cudaSuccess)
     cudaGetLastError();
   m->direct = direct != 0;
-  const size_t nx = direct ? 0 : round256(chunk * RH_MLP_IN * 4),
-               nt = direct ? 0 : round256(B * RH_MLP_OUT * 4),
-               no = round256(2 * chunk * RH_MLP_OUT * 4), ng = round256(kNPar * 4);
+  const size_t no = round256(2 * chunk * RH_MLP_OUT * 4), ng = round256(kNPar * 4);
   if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreate(&m->st) != cudaSuccess ||
       cudaMalloc(&m->P, (3 + parts) * (size_t)kNPar * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&m->img, kImgBytes) != cudaSuccess ||
-      cudaHostAlloc(&m->host, 2 * nx + nt + no + ng + 256, cudaHostAllocMapped) != cudaSuccess ||
+      cudaHostAlloc(&m->host, no + ng + 256, cudaHostAllocMapped) != cudaSuccess ||
       cudaEventCreateWithFlags(&m->ev[0], cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&m->ev[1], cudaEventDisableTiming) != cudaSuccess ||
       cudaFuncSetAttribute(mlp_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -960,11 +970,9 @@ int rh_mlp_create(int32_t batch_max, int32_t device, rh_mlp** out) {
   m->m = m->w + kNPar;
   m->v = m->m + kNPar;
   m->part = m->v + kNPar;
-  m->h_x = reinterpret_cast<float*>(m->host);  // two chunks
-  m->h_t = reinterpret_cast<float*>(m->host + 2 * nx);
-  m->h_out = reinterpret_cast<float*>(m->host + 2 * nx + nt);
-  m->h_g = reinterpret_cast<float*>(m->host + 2 * nx + nt + no);
-  m->h_err = reinterpret_cast<int*>(m->host + 2 * nx + nt + no + ng);
+  m->h_out = reinterpret_cast<float*>(m->host);
+  m->h_g = reinterpret_cast<float*>(m->host + no);
+  m->h_err = reinterpret_cast<int*>(m->host + no + ng);
   *m->h_err = 0;
   *out = m;
   return RH_OK;
@@ -976,6 +984,7 @@ int rh_mlp_destroy(rh_mlp* m) {
   cudaFree(m->P);
   cudaFree(m->img);
   if (m->host) cudaFreeHost(m->host);
+  if (m->copies) cudaFreeHost(m->copies);
   for (cudaEvent_t e : m->ev)
     if (e) cudaEventDestroy(e);
   if (m->st) cudaStreamDestroy(m->st);
@@ -1021,8 +1030,9 @@ int rh_mlp_forward(rh_mlp* m, const float* x, int32_t n, float* y) {
     RowsArgs a{};
     a.img = m->img;
     a.params = m->w;
-    a.x = reachable(m, x + (size_t)c * C * RH_MLP_IN, (size_t)rows(c) * RH_MLP_IN,
-                    m->h_x + (size_t)(c & 1) * C * RH_MLP_IN);
+    const int rx = reachable(m, x + (size_t)c * C * RH_MLP_IN, (size_t)rows(c) * RH_MLP_IN,
+                             c & 1 ? kCopyX1 : kCopyX0, &a.x);
+    if (rx != RH_OK) return rx;
     a.y = buffer(c);
     a.n = rows(c);
     a.err = m->h_err;
