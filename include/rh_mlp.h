@@ -47,6 +47,17 @@ int rh_mlp_train_step(rh_mlp* m, const float* x, const float* target, int32_t n,
                       float* loss);
 int rh_mlp_last_error(const rh_mlp* m, char* buf, size_t n);
 
+/* Check of the library's GEMM kernels (testing aid; synchronous, default
+ * stream): C[M x N] (FP32, row-major, leading dimension ldc) = sum over k of
+ * A(m, k) B(k, n), with A(m, k) = A[m*sam + k*sak] and B(k, n) =
+ * B[k*sbk + n*sbn] BF16 device arrays and C a device array; N <= 128.
+ * tensor_cores = 1 runs the tcgen05 kernel (tensor-memory accumulator; the
+ * general-stride form of the products in the network's own kernel), 0 the
+ * mma.sync kernel kept as its independent check. */
+int rh_mlp_gemm_check(const void* A, int32_t sam, int32_t sak, const void* B, int32_t sbk,
+                      int32_t sbn, float* C, int32_t ldc, int32_t M, int32_t N, int32_t K,
+                      int32_t tensor_cores);
+
 /* Forward pass that allocates nothing.  It has no counterpart in the
  * reference.  It is for callers that may not call cudaMalloc themselves or
  * have the library call it: programs whose device memory belongs to their own
@@ -62,20 +73,12 @@ int rh_mlp_last_error(const rh_mlp* m, char* buf, size_t n);
  *
  * The intermediate values live in the kernel's shared memory: the library
  * keeps no array for them, and calls on different streams or threads are
- * independent.  The first call on a device sets the kernel up (once, by the
- * runtime); make it before any stream capture.  n above RH_MLP_NOALLOC_MAX_BATCH is rejected with RH_ERR_ARG
- * and a message in err (err may be NULL). */
-/* Check of the library's GEMM kernels (testing aid; synchronous, default
- * stream): C[M x N] (FP32, row-major, leading dimension ldc) = sum over k of
- * A(m, k) B(k, n), with A(m, k) = A[m*sam + k*sak] and B(k, n) =
- * B[k*sbk + n*sbn] BF16 device arrays and C a device array; N <= 128.
- * tensor_cores = 1 runs the tcgen05 kernel (tensor-memory accumulator; the
- * general-stride form of the products in the network's own kernel), 0 the
- * mma.sync kernel kept as its independent check. */
-int rh_mlp_gemm_check(const void* A, int32_t sam, int32_t sak, const void* B, int32_t sbk,
-                      int32_t sbn, float* C, int32_t ldc, int32_t M, int32_t N, int32_t K,
-                      int32_t tensor_cores);
-
+ * independent.  d_y may overlap d_x or d_params: the call reads all of both
+ * before it writes (more than 128 samples then run on at most eight SMs).
+ * The first call on a device sets the kernels up (once, by the runtime); make
+ * it, with and without overlap if you need both, before any stream capture.
+ * n above RH_MLP_NOALLOC_MAX_BATCH is rejected with RH_ERR_ARG and a message
+ * in err (err may be NULL). */
 #define RH_MLP_NOALLOC_MAX_BATCH 4096
 #define RH_MLP_NOALLOC_SCRATCH_BYTES 0 /* device memory the library holds for it */
 int rh_mlp_forward_noalloc(const float* d_params, const float* d_x, int32_t n, float* d_y,
