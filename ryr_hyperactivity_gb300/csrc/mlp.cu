@@ -353,6 +353,7 @@ struct RowsArgs {
   float* part;               // [gridDim.x][kNPar] gradients (training)
   int n;
   int* err;                  // set when a wait gave up; nullptr: y becomes NaN
+  int* failed;               // the same for mlp_finish, in device memory (training)
 };
 
 // One MMA chain: K = 16 ksteps, descriptors advancing by da and db bytes.
@@ -731,6 +732,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) mlp_rows(const RowsArgs a) {
   }
   if (!done) {
     if (tid == 0 && a.err) *a.err = 1;  // host memory, read after a synchronisation
+    if (TRAIN && tid == 0) *a.failed = 1;
     if (!TRAIN && !a.err)
       for (int t = blockIdx.x; t < tiles; t += gridDim.x)
         for (int i = tid; i < 128 * RH_MLP_OUT; i += kRowThreads)
@@ -788,12 +790,13 @@ __global__ void __launch_bounds__(kRowThreads, 1) mlp_rows(const RowsArgs a) {
 
 // What follows a training pass: the CTAs' gradients added in order, then
 // either written out or taken as one Adam step on the FP32 master weights,
-// refreshing the BF16 image.  Padding weights stay zero.
+// refreshing the BF16 image.  Padding weights stay zero.  After a pass whose
+// wait gave up (`failed`), whose CTA has left no gradients, no step is taken.
 struct AdamStep {
   float lr, b1, b2, eps, bc1, bc2;
 };
 __global__ void mlp_finish(const float* part, int nparts, float* grads, float* w, float* m, float* v,
-                           unsigned char* img, AdamStep s) {
+                           unsigned char* img, const int* failed, AdamStep s) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= kNPar) return;
   float gi = 0.f;
@@ -804,11 +807,13 @@ __global__ void mlp_finish(const float* part, int nparts, float* grads, float* w
   }
   const ParamPlace p = place_of(i);
   if (p.padded) return;
+  const bool none = *failed != 0;  // read beside the moments, whose latency hides it
   const float mi = s.b1 * m[i] + (1.f - s.b1) * gi;
   const float vi = s.b2 * v[i] + (1.f - s.b2) * gi * gi;
+  const float wi = w[i] - s.lr * (mi / s.bc1) / (sqrtf(vi / s.bc2) + s.eps);
+  if (none) return;
   m[i] = mi;
   v[i] = vi;
-  const float wi = w[i] - s.lr * (mi / s.bc1) / (sqrtf(vi / s.bc2) + s.eps);
   w[i] = wi;
   if (p.img >= 0) *reinterpret_cast<__nv_bfloat16*>(img + p.img) = __float2bfloat16(wi);
 }
@@ -837,13 +842,14 @@ struct rh_mlp {
   cudaStream_t st = nullptr;
   float* P = nullptr;            // w, m, v, then the CTAs' gradients
   float *w = nullptr, *m = nullptr, *v = nullptr, *part = nullptr;
-  unsigned char* img = nullptr;  // BF16 weights (kImgBytes)
+  unsigned char* img = nullptr;  // BF16 weights (kImgBytes), then `failed`
   // Host memory the kernels read and write directly (pinned, mapped): outputs
   // of two chunks or loss terms, gradients, the error flag; and, made when first
   // needed, copies of the caller's arrays (reachable(), below).
   unsigned char* host = nullptr;
   float *h_out = nullptr, *h_g = nullptr, *copies = nullptr;
   int* h_err = nullptr;          // set by a pass whose wait gave up
+  int* failed = nullptr;         // and its copy for mlp_finish, on the device
   cudaEvent_t ev[2] = {nullptr, nullptr};
   bool direct = false;  // kernels can read pageable host memory (hardware page tables)
   int chunk = 0;        // samples of one forward launch
@@ -868,6 +874,7 @@ int ck(rh_mlp* m, cudaError_t e, const char* what) {
 int check_wait(rh_mlp* m) {
   if (*m->h_err) {
     *m->h_err = 0;
+    MCK(cudaMemsetAsync(m->failed, 0, sizeof(int), m->st));
     m->err = "a wait for the tensor cores ran out";
     return RH_ERR_TIMEOUT;
   }
@@ -915,6 +922,7 @@ int train_pass(rh_mlp* m, const float* x, const float* target, int n, int* npart
   a.part = m->part;
   a.n = n;
   a.err = m->h_err;
+  a.failed = m->failed;
   mlp_rows<true><<<*nparts, kRowThreads, RowsSmem::bytes(true), m->st>>>(a);
   return ck(m, cudaGetLastError(), "training pass");
 }
@@ -974,7 +982,7 @@ int rh_mlp_create(int32_t batch_max, int32_t device, rh_mlp** out) {
   const size_t no = round256(2 * chunk * RH_MLP_OUT * 4), ng = round256(kNPar * 4);
   if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreate(&m->st) != cudaSuccess ||
       cudaMalloc(&m->P, (3 + parts) * (size_t)kNPar * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&m->img, kImgBytes) != cudaSuccess ||
+      cudaMalloc(&m->img, kImgBytes + 256) != cudaSuccess ||
       cudaHostAlloc(&m->host, no + ng + 256, cudaHostAllocMapped) != cudaSuccess ||
       cudaEventCreateWithFlags(&m->ev[0], cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&m->ev[1], cudaEventDisableTiming) != cudaSuccess ||
@@ -983,7 +991,7 @@ int rh_mlp_create(int32_t batch_max, int32_t device, rh_mlp** out) {
       cudaFuncSetAttribute(mlp_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            RowsSmem::bytes(false)) != cudaSuccess ||
       cudaMemset(m->P, 0, 3 * (size_t)kNPar * sizeof(float)) != cudaSuccess ||
-      cudaMemset(m->img, 0, kImgBytes) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+      cudaMemset(m->img, 0, kImgBytes + 256) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
     m->err = "allocation failed";
     cudaGetLastError();
     rh_mlp_destroy(m);
@@ -993,6 +1001,7 @@ int rh_mlp_create(int32_t batch_max, int32_t device, rh_mlp** out) {
   m->m = m->w + kNPar;
   m->v = m->m + kNPar;
   m->part = m->v + kNPar;
+  m->failed = reinterpret_cast<int*>(m->img + kImgBytes);
   m->h_out = reinterpret_cast<float*>(m->host);
   m->h_g = reinterpret_cast<float*>(m->host + no);
   m->h_err = reinterpret_cast<int*>(m->host + no + ng);
@@ -1088,7 +1097,7 @@ int rh_mlp_gradients(rh_mlp* m, const float* x, const float* target, int32_t n, 
   if (r) return r;
   if (grads) {
     mlp_finish<<<blocks(kNPar, 256), 256, 0, m->st>>>(m->part, parts, m->h_g, nullptr, nullptr,
-                                                      nullptr, nullptr, AdamStep{});
+                                                      nullptr, nullptr, m->failed, AdamStep{});
     r = ck(m, cudaGetLastError(), "gradients");
   }
   const int rs = ck(m, cudaStreamSynchronize(m->st), "gradients");
@@ -1106,16 +1115,17 @@ int rh_mlp_train_step(rh_mlp* m, const float* x, const float* target, int32_t n,
   int parts = 0;
   int r = train_pass(m, x, target, n, &parts);
   if (r) return r;
-  m->step += 1;
+  const float step = (float)(m->step + 1);
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  const AdamStep s{lr, b1, b2, eps, 1.f - powf(b1, (float)m->step), 1.f - powf(b2, (float)m->step)};
+  const AdamStep s{lr, b1, b2, eps, 1.f - powf(b1, step), 1.f - powf(b2, step)};
   mlp_finish<<<blocks(kNPar, 256), 256, 0, m->st>>>(m->part, parts, nullptr, m->w, m->m, m->v,
-                                                    m->img, s);
+                                                    m->img, m->failed, s);
   r = ck(m, cudaGetLastError(), "training step");
   const int rs = ck(m, cudaStreamSynchronize(m->st), "training step");
   if (r) return r;
   if (rs) return rs;
   if ((r = check_wait(m))) return r;
+  m->step += 1;
   if (loss) *loss = mean_loss(m, n);
   return RH_OK;
 }
