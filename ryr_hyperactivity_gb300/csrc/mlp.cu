@@ -95,7 +95,8 @@ __global__ void gemm_bf16(const __nv_bfloat16* __restrict__ A, int sam, int sak,
 // they have read shared memory.  Each warp then reads its 32 accumulator
 // rows with tcgen05.ld and writes C.  Out-of-range elements read as zero.
 // Every wait on the mbarrier is bounded: on expiry the CTA sets *err, skips
-// the rest of its MMAs and still frees its tensor memory.
+// the rest of its MMAs, waits once more (bounded again) for those in flight and
+// frees its tensor memory.
 namespace tc {
 
 constexpr int kM = 128;   // rows per CTA = tensor-memory lanes
@@ -103,7 +104,9 @@ constexpr int kKc = 128;  // K elements per staged chunk
 constexpr int kNmax = 128;
 constexpr int kSmemA = kM * kKc * 2;      // bytes
 constexpr int kSmemB = kNmax * kKc * 2;
-constexpr long long kWaitLimit = 1 << 22;  // polls of an mbarrier (a few ms)
+// Polls of an mbarrier before a wait gives up: the hardware holds a poll for up
+// to 3.75 us while nothing arrives (2^22 of them took 15.7 s), so 1 s in all.
+constexpr int kWaitLimit = 1 << 18;
 
 __device__ __forceinline__ uint32_t saddr(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -132,7 +135,7 @@ __device__ __forceinline__ uint32_t core_off(int row, int k, int rows) {
 }
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  for (long long it = 0; it < kWaitLimit; ++it) {
+  for (int it = 0; it < kWaitLimit; ++it) {
     uint32_t done;
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
@@ -182,7 +185,8 @@ __global__ void __launch_bounds__(128, 1)
   const uint32_t idesc = tc::instr_desc(tc::kM, Nm);
   bool ok = true;
   const int nchunks = (K + tc::kKc - 1) / tc::kKc;
-  for (int ch = 0; ch < nchunks && ok; ++ch) {
+  int ch = 0;
+  for (; ch < nchunks && ok; ++ch) {
     const int k0 = ch * tc::kKc;
     // stage A (128 x 128) and B (Nm x 128) as 16-byte core-matrix rows
     for (int c = tid; c < tc::kM * (tc::kKc / 8); c += blockDim.x) {
@@ -242,6 +246,7 @@ __global__ void __launch_bounds__(128, 1)
   }
   if (!ok) {
     if (tid == 0) atomicOr(err, 1);
+    tc::mbar_wait(tc::saddr(&bar), (uint32_t)((ch - 1) & 1));  // the last commit's phase
   } else {
     // epilogue: warp w reads accumulator rows 32w..32w+31 (its tensor-memory lanes)
     const int row = m0 + warp * 32 + lane;
@@ -733,6 +738,11 @@ __global__ void __launch_bounds__(kRowThreads, 1) mlp_rows(const RowsArgs a) {
   if (!done) {
     if (tid == 0 && a.err) *a.err = 1;  // host memory, read after a synchronisation
     if (TRAIN && tid == 0) *a.failed = 1;
+    // nothing may still write this CTA's shared or tensor memory when it ends:
+    // the weights' copy, the last MMAs committed (if none were, the phase
+    // before the first counts as complete)
+    if (a.img) tc::mbar_wait(w_bar, 0);
+    tc::mbar_wait(mma_bar, phase ^ 1u);
     if (!TRAIN && !a.err)
       for (int t = blockIdx.x; t < tiles; t += gridDim.x)
         for (int i = tid; i < 128 * RH_MLP_OUT; i += kRowThreads)

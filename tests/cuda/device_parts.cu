@@ -78,6 +78,13 @@ __global__ void divide_kernel(int n, const double* a, const double* b, double* q
   if (i < n) q[i] = div_refined(a[i], b[i]);
 }
 
+__global__ void wait_kernel(int* gave_up) {
+  __shared__ __align__(8) uint64_t bar;
+  if (threadIdx.x == 0) mbar_init(&bar, 1);
+  __syncthreads();
+  if (!mbar_wait(&bar, 0)) *gave_up = 1;  // nothing ever arrives
+}
+
 }  // namespace
 
 extern "C" {
@@ -124,6 +131,15 @@ int part_divide(int n, const double* a, const double* b, double* q) {
   Dev<double> da(a, (size_t)n), db(b, (size_t)n), dq(nullptr, (size_t)n);
   divide_kernel<<<(n + 127) / 128, 128>>>(n, da.p, db.p, dq.p);
   return dq.get(q) ? 0 : -1;
+}
+
+// 1 when a wait for an arrival that never comes has given up
+int part_wait_runs_out() {
+  const int zero = 0;
+  Dev<int> d(&zero, 1);
+  wait_kernel<<<1, 32>>>(d.p);
+  int h = -1;
+  return d.get(&h) ? h : -1;
 }
 
 }  // extern "C"

@@ -1,11 +1,19 @@
 // A training step whose pass reports a wait that gave up: the flags it would
 // set are set by hand before the step.  The step fails, and parameters,
 // moments and step count stay as they were: the next step gives what it gives
-// without the failed one.
+// without the failed one.  And a wait for an arrival that never comes, by itself.
 // Build: nvcc -gencode arch=compute_103a,code=sm_103a -std=c++17
 #include "../../ryr_hyperactivity_gb300/csrc/mlp.cu"
 
 #include <vector>
+
+__global__ void wait_kernel(int* gave_up) {
+  __shared__ __align__(8) uint64_t bar;
+  if (threadIdx.x == 0)
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc::saddr(&bar)) : "memory");
+  __syncthreads();
+  if (!tc::mbar_wait(tc::saddr(&bar), 0)) *gave_up = 1;  // nothing ever arrives
+}
 
 int main() {
   constexpr int n = 300;
@@ -33,6 +41,19 @@ int main() {
   const bool same = !memcmp(a.data(), b.data(), kNPar * sizeof(float));
   const bool moved = memcmp(a.data(), before.data(), kNPar * sizeof(float)) != 0;
   printf("timeout %d kept %d same %d moved %d\n", rc == RH_ERR_TIMEOUT, kept, same, moved);
+  int *flag = nullptr, gave_up = 0;
+  float ms = 0;
+  cudaEvent_t e0, e1;
+  cudaEventCreate(&e0);
+  cudaEventCreate(&e1);
+  if (cudaMalloc(&flag, sizeof(int)) != cudaSuccess || cudaMemset(flag, 0, sizeof(int)) != cudaSuccess)
+    return 9;
+  cudaEventRecord(e0);
+  wait_kernel<<<1, 512>>>(flag);
+  cudaEventRecord(e1);
+  if (cudaMemcpy(&gave_up, flag, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return 10;
+  cudaEventElapsedTime(&ms, e0, e1);
+  printf("wait gave up %d within 3 s %d (%.0f ms)\n", gave_up, ms < 3000.f, ms);
   rh_mlp_destroy(u);
   rh_mlp_destroy(w);
   return 0;

@@ -156,3 +156,11 @@ def test_refined_division_equals_the_rounded_quotient(parts, kind):
         want = a / b
     bad = (q.view(np.uint64) != want.view(np.uint64)) & ~(np.isnan(q) & np.isnan(want))
     assert not bad.any(), (int(bad.sum()), a[bad][:5], b[bad][:5], q[bad][:5], want[bad][:5])
+
+
+def test_a_wait_that_nothing_ends_gives_up_within_seconds(parts):
+    import time
+    parts.part_output_sums(_p(np.zeros((1, parts.part_row_length()))), 1, _p(np.zeros(64)))
+    t = time.perf_counter()
+    assert parts.part_wait_runs_out() == 1
+    assert time.perf_counter() - t < 3.0

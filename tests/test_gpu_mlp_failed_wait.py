@@ -15,4 +15,6 @@ def test_a_failed_step_leaves_the_model_unchanged(tmp_path):
                     os.path.join(ROOT, "include"),
                     os.path.join(ROOT, "tests", "cuda", "mlp_failed_wait.cu"), "-o", exe], check=True)
     out = subprocess.run([exe], check=True, capture_output=True, text=True).stdout
-    assert out.strip() == "timeout 1 kept 1 same 1 moved 1"
+    lines = out.splitlines()
+    assert lines[0] == "timeout 1 kept 1 same 1 moved 1"
+    assert lines[1].startswith("wait gave up 1 within 3 s 1")
