@@ -31,6 +31,8 @@ extern "C" {
 
 typedef struct rh_mlp rh_mlp;
 
+/* batch_max: largest batch of rh_mlp_gradients and rh_mlp_train_step; above
+ * 2^26 samples RH_ERR_NOMEM. */
 int rh_mlp_create(int32_t batch_max, int32_t device, rh_mlp** out);
 int rh_mlp_destroy(rh_mlp* m);
 int rh_mlp_param_count(const rh_mlp* m, int32_t* n);

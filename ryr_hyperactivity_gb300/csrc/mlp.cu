@@ -845,6 +845,9 @@ unsigned blocks(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 constexpr int kChunk = 16384;    // samples of one forward launch
 constexpr int kMaxParts = 152;   // CTAs of a training pass
+// Largest batch of a handle: more pinned memory (24 bytes a sample) than that is
+// no screening network's, and sample indices stay far from overflow.
+constexpr int kMaxBatch = 1 << 26;
 
 struct rh_mlp {
   int bmax = 0;
@@ -977,6 +980,7 @@ int rh_mlp_gemm_check(const void* A, int32_t sam, int32_t sak, const void* B, in
 int rh_mlp_create(int32_t batch_max, int32_t device, rh_mlp** out) {
   if (!out || batch_max <= 0) return RH_ERR_ARG;
   *out = nullptr;
+  if (batch_max > kMaxBatch) return RH_ERR_NOMEM;
   rh_mlp* m = new rh_mlp();
   m->bmax = batch_max;
   m->device = device;

@@ -55,3 +55,11 @@ def test_gradients_and_steps_take_arrays_at_any_address(n, by):
         m.set_params(_off(m.get_params(), by))
     np.testing.assert_array_equal(a.get_params(), b.get_params())
     assert not np.array_equal(a.get_params(), init_params(2))
+
+
+@pytest.mark.parametrize("batch_max", [(1 << 26) + 1, (1 << 31) - 1])
+def test_a_batch_no_memory_holds_is_refused(batch_max):
+    from ryr_hyperactivity_gb300.surrogate import _lib
+    h = C.c_void_p()
+    assert _lib().rh_mlp_create(batch_max, 0, C.byref(h)) == -3  # RH_ERR_NOMEM
+    assert not h.value
