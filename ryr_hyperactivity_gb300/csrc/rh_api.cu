@@ -1694,6 +1694,77 @@ int rh_tile_size(const rh_sim* s, int32_t* tile) {
   return RH_OK;
 }
 
+}  // extern "C"
+
+namespace {
+
+// Times steps of the current launch shape for the autotuners, from a copy of
+// the state on the device.  The steps run as those of a window do (two-launch
+// path: one graph with a branch per cell group): launched one by one, small
+// simulations would be timed by the host's launches (37 us a step of 50 small
+// cells that take 17).  They write no output records, so that records still
+// waiting in the output rings are never overwritten (one step in 100 is an
+// output step; its extra stores do not move the choice).
+struct Trial {
+  rh_sim* s;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  explicit Trial(rh_sim* sim) : s(sim) {
+    cudaEventCreate(&e0);
+    cudaEventCreate(&e1);
+  }
+  ~Trial() {
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+  }
+  void restore(const char* bk) {
+    cudaMemcpyAsync(s->arena, bk, s->arena_bytes, cudaMemcpyDeviceToDevice, s->stream);
+    cudaMemcpyAsync(s->d_dyn, bk + s->arena_bytes, sizeof(CellDyn) * (size_t)s->ncells,
+                    cudaMemcpyDeviceToDevice, s->stream);
+  }
+  cudaError_t capture(int n, cudaGraphExec_t* exec) {
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) return e;
+    std::unique_ptr<bool[]> outs(new bool[n]());
+    const cudaError_t le = launch_steps(s, n, outs.get(), false);
+    e = cudaStreamEndCapture(s->stream, &g);
+    if (le != cudaSuccess) e = le;
+    if (e == cudaSuccess)
+      e = cudaGraphInstantiate(exec, g, cudaGraphInstantiateFlagUseNodePriority);
+    if (g) cudaGraphDestroy(g);
+    return e;
+  }
+  // ms per step, after one untimed run of the same steps (whole windows from
+  // 100 steps on)
+  int time(const char* bk, int steps, double* ms_per_step) {
+    const int n = std::min(steps, 100), windows = (steps + n - 1) / n;
+    cudaGraphExec_t exec = nullptr;
+    cudaError_t e = use_persist(s) ? cudaSuccess : capture(n, &exec);
+    for (int pass = 0; pass < 2 && e == cudaSuccess; ++pass) {
+      restore(bk);
+      cudaEventRecord(e0, s->stream);
+      for (int w = 0; w < windows && e == cudaSuccess; ++w)
+        e = exec ? cudaGraphLaunch(exec, s->stream) : launch_persist(s, n, true);
+      cudaEventRecord(e1, s->stream);
+    }
+    if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+    if (exec) cudaGraphExecDestroy(exec);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return fail(s, RH_ERR_CUDA, "autotune: %s", cudaGetErrorString(e));
+    }
+    const int r = check_wait_error(s);
+    float ms = 0;
+    cudaEventElapsedTime(&ms, e0, e1);
+    *ms_per_step = (double)ms / n / windows;
+    return r;
+  }
+};
+
+}  // namespace
+
+extern "C" {
+
 int rh_autotune(rh_sim* s, int32_t steps, int32_t* tile, double* ms_per_step) {
   if (!s || steps <= 0) return RH_ERR_ARG;
   CK(cudaSetDevice(s->device));
@@ -1715,40 +1786,12 @@ int rh_autotune(rh_sim* s, int32_t steps, int32_t* tile, double* ms_per_step) {
   s->shape_given = true;
   double best = 1e300;
   int best_k = ts0;
-  cudaEvent_t e0, e1;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
+  Trial trial(s);
   int rc = RH_OK;
   for (int k = 0; k < kNumTileSizes && rc == RH_OK; ++k) {
     s->ts = k;
-    cudaMemcpyAsync(s->arena, bk, s->arena_bytes, cudaMemcpyDeviceToDevice, s->stream);
-    cudaMemcpyAsync(s->d_dyn, bk + s->arena_bytes, dyn_bytes, cudaMemcpyDeviceToDevice, s->stream);
-    cudaEventRecord(e0, s->stream);
-    // the trial steps write no output records, so records still waiting in
-    // the output rings are never overwritten (one step in 100 is an output
-    // step; its extra stores do not move the choice)
-    if (use_persist(s)) {  // one persistent launch of `steps` steps
-      cudaError_t e = launch_persist(s, steps, true);
-      if (e != cudaSuccess) rc = fail(s, RH_ERR_CUDA, "autotune launch: %s", cudaGetErrorString(e));
-    } else {
-      for (int i = 0; i < steps; ++i) {  // the output-free kernel variant
-        cudaError_t e = launch_one(s, false, false);
-        if (e != cudaSuccess) {
-          rc = fail(s, RH_ERR_CUDA, "autotune launch: %s", cudaGetErrorString(e));
-          break;
-        }
-      }
-    }
-    if (rc != RH_OK) break;
-    cudaEventRecord(e1, s->stream);
-    if (cudaEventSynchronize(e1) != cudaSuccess) {
-      rc = fail(s, RH_ERR_CUDA, "autotune: %s", cudaGetErrorString(cudaGetLastError()));
-      break;
-    }
-    if ((rc = check_wait_error(s)) != RH_OK) break;
-    float ms = 0;
-    cudaEventElapsedTime(&ms, e0, e1);
-    double per = ms / steps;
+    double per = 0;
+    if ((rc = trial.time(bk, steps, &per)) != RH_OK) break;
     if (ms_per_step) ms_per_step[k] = per;
     if (per < best) {
       best = per;
@@ -1756,12 +1799,9 @@ int rh_autotune(rh_sim* s, int32_t steps, int32_t* tile, double* ms_per_step) {
     }
   }
   // restore the state and select the winner
-  cudaMemcpyAsync(s->arena, bk, s->arena_bytes, cudaMemcpyDeviceToDevice, s->stream);
-  cudaMemcpyAsync(s->d_dyn, bk + s->arena_bytes, dyn_bytes, cudaMemcpyDeviceToDevice, s->stream);
+  trial.restore(bk);
   cudaStreamSynchronize(s->stream);
   cudaFree(backup);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
   s->t_host = t0;
   s->active_host = a0;
   s->ts = rc == RH_OK ? best_k : ts0;
@@ -1942,42 +1982,14 @@ int rh_autotune_shapes(rh_sim* s, int32_t steps, rh_launch_shape* best,
   CK(cudaMemcpyAsync(bk + s->arena_bytes, s->d_dyn, dyn_bytes, cudaMemcpyDeviceToDevice, s->stream));
   const std::vector<double> t0 = s->t_host;
   const std::vector<char> a0 = s->active_host;
-  auto restore = [&]() {
-    cudaMemcpyAsync(s->arena, bk, s->arena_bytes, cudaMemcpyDeviceToDevice, s->stream);
-    cudaMemcpyAsync(s->d_dyn, bk + s->arena_bytes, dyn_bytes, cudaMemcpyDeviceToDevice, s->stream);
-  };
-  cudaEvent_t e0, e1;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
-  // the trial steps write no output records (see rh_autotune)
-  auto trial = [&](int n) -> cudaError_t {
-    if (use_persist(s)) return launch_persist(s, n, true);
-    for (int i = 0; i < n; ++i) {
-      cudaError_t e = launch_one(s, false, false);
-      if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
-  };
+  Trial trial(s);
   int rc = RH_OK, nt = 0;
   double best_ms = 1e300;
   rh_launch_shape win = orig;
   for (const rh_launch_shape& c : cand) {
     if (rh_set_launch_shape(s, &c) != RH_OK) continue;
-    restore();
-    cudaError_t e = trial(std::max(1, steps / 4));  // first launches of this shape, untimed
-    restore();
-    cudaEventRecord(e0, s->stream);
-    if (e == cudaSuccess) e = trial(steps);
-    cudaEventRecord(e1, s->stream);
-    if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-    if (e != cudaSuccess) {
-      rc = fail(s, RH_ERR_CUDA, "autotune: %s", cudaGetErrorString(e));
-      break;
-    }
-    if ((rc = check_wait_error(s)) != RH_OK) break;
-    float ms = 0;
-    cudaEventElapsedTime(&ms, e0, e1);
-    const double per = ms / steps;
+    double per = 0;
+    if ((rc = trial.time(bk, steps, &per)) != RH_OK) break;
     if (nt < max_tried) {
       if (tried) tried[nt] = c;
       if (ms_per_step) ms_per_step[nt] = per;
@@ -1988,11 +2000,9 @@ int rh_autotune_shapes(rh_sim* s, int32_t steps, rh_launch_shape* best,
       win = c;
     }
   }
-  restore();
+  trial.restore(bk);
   cudaStreamSynchronize(s->stream);
   cudaFree(backup);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
   s->t_host = t0;
   s->active_host = a0;
   if (ntried) *ntried = std::min(nt, max_tried);
