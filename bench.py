@@ -272,7 +272,7 @@ def main():
     else:  # launch shape for this workload (the simulation state is unchanged)
         _, tune = sim.autotune_shapes(40)
     shape = sim.launch_shape()
-    tile = shape["tile_crus"]
+    tile = sim.tile_size()
     sim.kernel_timing()  # reset
     sim.drain_wholecell_all()
     kernels0, persistent = sim.kernel_launches()

@@ -314,10 +314,14 @@ int rh_run_steps_host(rh_sim* sim, int64_t nsteps, const void* host_in, void* ho
  * register/occupancy bound).  Times `steps` lattice updates of the live
  * workload with each candidate, starting every candidate from a device-side
  * copy of the current state and restoring that state afterwards (the
- * simulation does not advance), then keeps the fastest.  ms_per_step (3
- * entries, may be NULL) receives the timings.  rh_autotune_shapes searches
- * the launch mode, CTAs per SM and cell groups as well. */
+ * simulation does not advance), then keeps the fastest, which *tile_crus and
+ * ms_per_step (3 entries, may be NULL) tell.  Of a small lattice the library's
+ * own choice (rh_launch_shape, tile_crus 0) is timed too and kept where it is
+ * faster than all three.  rh_autotune_shapes searches the launch mode, CTAs
+ * per SM and cell groups as well. */
 int rh_autotune(rh_sim* sim, int32_t steps, int32_t* tile_crus, double* ms_per_step);
+/* CRUs per CTA of the lattice updates as they are launched now: 64, 128, 256,
+ * or 32 where the library chose narrow tiles by itself. */
 int rh_tile_size(const rh_sim* sim, int32_t* tile_crus);
 
 /* How the time steps of a simulator are launched: the autotuner's search
@@ -328,10 +332,13 @@ typedef struct {
   int32_t persistent;   /* 1 = one persistent cooperative launch per window,
                            0 = two launches per step and cell group */
   int32_t tile_crus;    /* CRUs (threads) per CTA: 64, 128 or 256; the
-                           persistent launch takes 64 or 128.  While no shape
-                           was asked for (block_size 0, no rh_set_launch_shape
-                           or autotuner), small lattices run one-warp CTAs
-                           instead, with the same results */
+                           persistent launch takes 64 or 128.  0 = the library's
+                           own choice of tiles and staging on the two-launch
+                           path, as while no shape was asked for (block_size
+                           0): narrow 32-CRU tiles of small lattices, else 128
+                           CRUs; the same results.  rh_get_launch_shape says 0
+                           while narrow tiles run, which are no shape of their
+                           own */
   int32_t fewer_ctas;   /* persistent launch only: 1 = one resident CTA per SM
                            fewer than the step kernel holds, with more registers
                            per thread (cells without build options only) */
@@ -343,8 +350,8 @@ typedef struct {
                            on mbarriers); 2 = the tile's ci/cnsr pair planes and
                            its eight real planes arrive as 2-D tensor tiles
                            (cp.async.bulk.tensor, one thread), the rest as in 0.
-                           While no shape was asked for, large ensembles run 2,
-                           with the same results */
+                           With tile_crus 0 pass 0: large ensembles run 2 by the
+                           library's choice, with the same results */
 } rh_launch_shape;
 
 int rh_get_launch_shape(const rh_sim* sim, rh_launch_shape* shape);
@@ -358,8 +365,8 @@ int rh_set_launch_shape(rh_sim* sim, const rh_launch_shape* shape);
 /* Launch-shape autotuner.  Times `steps` lattice updates of the live
  * workload with every candidate shape (persistent launches with tiles of 64
  * and 128 at both CTA counts; two-launch windows with tiles of 64, 128 and
- * 256 at 8, 12, 16 and 24 cell groups, in mixed precision with each staging),
- * each from a device-side copy of the
+ * 256 at 8, 12, 16 and 24 cell groups, in mixed precision with each staging;
+ * the library's own choice, tile_crus 0, where it runs narrow tiles), each from a device-side copy of the
  * current state that is restored afterwards (the simulation does not
  * advance), and switches to the fastest.  The choice is cached for the
  * process by device, precision and lattice classes (the cells' interior x

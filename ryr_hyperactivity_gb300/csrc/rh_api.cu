@@ -46,6 +46,7 @@ struct rh_sim {
     int4* d_tiles = nullptr;
   } sets[kNumTileSets];
   int ts = 0;
+  int default_ts = 0;        // of kDefaultTile
   bool shape_given = false;  // a tile length was asked for (run option, launch shape, autotuner)
   int sm_count = 0;
   // Cell groups: contiguous cell ranges of about equal CRU count, each with
@@ -311,10 +312,12 @@ bool use_persist(const rh_sim* s) {
 // default).  FP32, up to the three split tiles an SM holds (narrow against
 // default tiles: one 100x20x10 cell 1.51 against 1.58 ms, two 80x16x8 cells
 // 1.40 against 1.44, 35 cells of 432 CRUs (490 tiles) 1.89 against 1.68).
-int active_set(const rh_sim* s) {
-  if (s->shape_given || use_persist(s)) return s->ts;
+bool small_lattice(const rh_sim* s) {
   const int64_t tiles_per_sm = is_mixed(s) ? kSplitBlocks : 12;
-  return s->sets[kNarrowSet].ntiles <= tiles_per_sm * s->sm_count ? kNarrowSet : s->ts;
+  return s->sets[kNarrowSet].ntiles <= tiles_per_sm * s->sm_count;
+}
+int active_set(const rh_sim* s) {
+  return s->shape_given || use_persist(s) || !small_lattice(s) ? s->ts : (int)kNarrowSet;
 }
 
 template <class R>
@@ -370,6 +373,14 @@ int lattice_staging(const rh_sim* s) {
   const int64_t wave = (int64_t)min_blocks_for<float, kDefaultTile>() * s->sm_count;
   const bool many = active_set(s) == s->ts && s->sets[s->ts].ntiles >= 3 * wave;
   return !s->shape_given && s->maps_ok && many ? 2 : s->staging;
+}
+
+// Gives the choice of tiles and staging on the two-launch path back to the
+// library (tile_crus 0).
+void choose_own(rh_sim* s) {
+  s->ts = s->default_ts;
+  s->shape_given = false;
+  s->staging = 0;
 }
 
 // One group's step: the tiles of cells [group_cell[g], group_cell[g+1]),
@@ -841,8 +852,10 @@ static int create_impl(rh_sim* s, const rh_cell_params* cells, int32_t ncells,
   {
     int want = s->opts.block_size > 0 ? s->opts.block_size : kDefaultTile;
     s->ts = -1;
-    for (int k = 0; k < kNumTileSizes; ++k)
+    for (int k = 0; k < kNumTileSizes; ++k) {
       if (kTileSizes[k] == want) s->ts = k;
+      if (kTileSizes[k] == kDefaultTile) s->default_ts = k;
+    }
     s->shape_given = s->opts.block_size > 0;
     if (s->ts < 0) return fail(s, RH_ERR_ARG, "block_size %d is not a compiled tile length", want);
   }
@@ -1690,7 +1703,7 @@ int rh_import_state(rh_sim* s, const void* host, size_t bytes) {
 
 int rh_tile_size(const rh_sim* s, int32_t* tile) {
   if (!s || !tile) return RH_ERR_ARG;
-  *tile = s->sets[s->ts].tile;
+  *tile = s->sets[active_set(s)].tile;
   return RH_OK;
 }
 
@@ -1705,6 +1718,9 @@ namespace {
 // cells that take 17).  They write no output records, so that records still
 // waiting in the output rings are never overwritten (one step in 100 is an
 // output step; its extra stores do not move the choice).
+//
+// The library's own choice of tiles is a candidate where it is not one of the
+// launch shapes, that is where it runs narrow tiles.
 struct Trial {
   rh_sim* s;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -1783,6 +1799,7 @@ int rh_autotune(rh_sim* s, int32_t steps, int32_t* tile, double* ms_per_step) {
   const std::vector<char> a0 = s->active_host;
   const int ts0 = s->ts;
   const bool given0 = s->shape_given;
+  const int staging0 = s->staging;
   s->shape_given = true;
   double best = 1e300;
   int best_k = ts0;
@@ -1798,6 +1815,12 @@ int rh_autotune(rh_sim* s, int32_t steps, int32_t* tile, double* ms_per_step) {
       best_k = k;
     }
   }
+  bool own = false;
+  if (rc == RH_OK && !s->opts.persistent && small_lattice(s)) {
+    choose_own(s);
+    double per = 0;
+    if ((rc = trial.time(bk, steps, &per)) == RH_OK) own = per < best;
+  }
   // restore the state and select the winner
   trial.restore(bk);
   cudaStreamSynchronize(s->stream);
@@ -1806,10 +1829,12 @@ int rh_autotune(rh_sim* s, int32_t steps, int32_t* tile, double* ms_per_step) {
   s->active_host = a0;
   s->ts = rc == RH_OK ? best_k : ts0;
   s->shape_given = rc == RH_OK || given0;
+  s->staging = staging0;
+  if (tile) *tile = s->sets[s->ts].tile;
+  if (own) choose_own(s);
   s->hcells = s->sets[s->ts].hcells;
   for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);
   s->graphs.clear();
-  if (tile) *tile = s->sets[s->ts].tile;
   CK(cudaGetLastError());
   return rc;
 }
@@ -1820,13 +1845,21 @@ int rh_get_launch_shape(const rh_sim* s, rh_launch_shape* shape) {
   shape->tile_crus = s->sets[s->ts].tile;
   shape->fewer_ctas = (shape->persistent && s->fewer_ctas) ? 1 : 0;
   shape->cell_groups = s->ngroups;
-  shape->bulk_staging = shape->persistent ? 0 : s->staging;
+  shape->bulk_staging = shape->persistent || !is_mixed(s) ? 0 : lattice_staging(s);
+  if (active_set(s) == kNarrowSet) {  // no launch shape: the library's own choice
+    shape->tile_crus = 0;
+    shape->bulk_staging = 0;
+  }
   return RH_OK;
 }
 
 int rh_set_launch_shape(rh_sim* s, const rh_launch_shape* shape) {
   if (!s || !shape) return RH_ERR_ARG;
-  int k = -1;
+  const bool own = shape->tile_crus == 0;
+  if (own && (shape->persistent || shape->bulk_staging))
+    return fail(s, RH_ERR_ARG, "the library's own choice (tile_crus 0) is one of the two-launch "
+                               "path, staging included");
+  int k = own ? s->default_ts : -1;
   for (int i = 0; i < kNumTileSizes; ++i)
     if (kTileSizes[i] == shape->tile_crus) k = i;
   if (k < 0) return fail(s, RH_ERR_NOTBUILT, "no kernel for tiles of %d CRUs", shape->tile_crus);
@@ -1849,7 +1882,7 @@ int rh_set_launch_shape(rh_sim* s, const rh_launch_shape* shape) {
   CK(cudaSetDevice(s->device));
   CK(cudaStreamSynchronize(s->stream));
   s->ts = k;
-  s->shape_given = true;
+  s->shape_given = !own;
   s->hcells = s->sets[k].hcells;
   s->opts.persistent = shape->persistent ? 1 : 0;
   s->fewer_ctas = shape->persistent && shape->fewer_ctas;
@@ -1881,7 +1914,8 @@ std::string workload_key(const rh_sim* s) {
   }
   std::string k = std::string(prop.name) + "|sm" + std::to_string(prop.multiProcessorCount) +
                   "|p" + std::to_string(s->opts.precision) + "|opt" +
-                  std::to_string(any_options(s) ? 1 : 0) + "|n" + std::to_string(crus);
+                  std::to_string(any_options(s) ? 1 : 0) + "|n" + std::to_string(crus) +
+                  (small_lattice(s) ? "|own" : "");  // another set of candidates
   for (const auto& kv : classes)
     k += "|" + std::to_string(kv.first.first) + "," + std::to_string(kv.first.second) + ":" +
          std::to_string(kv.second);
@@ -1958,6 +1992,7 @@ int rh_autotune_shapes(rh_sim* s, int32_t steps, rh_launch_shape* best,
   }
   // candidates
   std::vector<rh_launch_shape> cand;
+  if (small_lattice(s)) cand.push_back(rh_launch_shape{0, 0, 0, s->ngroups, 0});
   if (s->persist_ok)
     for (int tile : {64, 128})
       for (int fewer = 0; fewer < (any_options(s) ? 1 : 2); ++fewer)

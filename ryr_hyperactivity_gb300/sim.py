@@ -183,7 +183,9 @@ class Simulator:
 
     def autotune(self, steps: int = 50) -> tuple[int, list[float]]:
         """Picks the fastest tile length for this workload; returns it and the
-        measured ms per step of each candidate (64, 128, 256 CRUs)."""
+        measured ms per step of each candidate (64, 128, 256 CRUs).  Of a small
+        lattice the library's own narrow tiles are kept where they are faster
+        than all three (tile_size() is then 32)."""
         tile = C.c_int32()
         ms = (C.c_double * 3)()
         self._ck(self.L.rh_autotune(self.h, int(steps), C.byref(tile), ms))
@@ -230,6 +232,8 @@ class Simulator:
 
     def set_launch_shape(self, persistent: int, tile_crus: int, fewer_ctas: int = 0,
                          cell_groups: int = 0, bulk_staging: int = 0) -> None:
+        """Takes what launch_shape() returns; tile_crus 0 leaves tiles and
+        staging to the library."""
         sh = LaunchShape(persistent, tile_crus, fewer_ctas, cell_groups, bulk_staging)
         self._ck(self.L.rh_set_launch_shape(self.h, C.byref(sh)))
 
