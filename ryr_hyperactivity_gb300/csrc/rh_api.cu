@@ -307,13 +307,16 @@ bool use_persist(const rh_sim* s) {
 // tiles (32 CRUs per CTA) where no shape was asked for and the lattice is
 // small.  128-CRU tiles then leave SMs without work: a 100x20x10 cell fills
 // 111 of 152.  FP64, up to 12 tiles per SM, the warps an SM holds: a warp's
-// rate is set by its scheduler's FP64 unit, so warps want spreading (per 100
-// steps: 1,350 tiles 10.1 ms, but 2,700 tiles 19.9 ms against 19.2 with the
-// default).  FP32, up to the three split tiles an SM holds (narrow against
-// default tiles: one 100x20x10 cell 1.51 against 1.58 ms, two 80x16x8 cells
-// 1.40 against 1.44, 35 cells of 432 CRUs (490 tiles) 1.89 against 1.68).
+// rate is set by its scheduler's FP64 unit, so warps want spreading (narrow
+// against default tiles, 100 steps: 1,260 tiles of 432-CRU cells 9.19 and 11.58
+// ms, 1,820 tiles 12.90 and 13.87, but 2,240 tiles 15.61 and 15.42).  FP32, up
+// to the three split tiles an SM holds (one 100x20x10 cell, 441 tiles, 1.32 and
+// 1.40 ms, two 80x16x8 cells, 410, 1.34 and 1.40; 539 tiles 1.89 and 1.41), with
+// more than two cell groups up to two: their launches fill a wave between them
+// (20 cells of 432 CRUs, 280 tiles, 1.52 and 1.55; 25 cells, 350, 1.59 and 1.56;
+// 30 cells, 420, 1.70 and 1.55).
 bool small_lattice(const rh_sim* s) {
-  const int64_t tiles_per_sm = is_mixed(s) ? kSplitBlocks : 12;
+  const int64_t tiles_per_sm = !is_mixed(s) ? 12 : s->ngroups > 2 ? 2 : kSplitBlocks;
   return s->sets[kNarrowSet].ntiles <= tiles_per_sm * s->sm_count;
 }
 int active_set(const rh_sim* s) {
@@ -346,28 +349,32 @@ StepArgs<R> make_args(rh_sim* s, const Lattice<R>& L, bool lattice_only) {
 // holds at most ten warps per SM, half of what an SM has room for, the cell
 // update is the step's critical path and its CTAs find room beside the
 // lattice's.  Four-warp against one-warp updates, per 100 steps: 50 cells of
-// 432 CRUs (5 warps per SM) 1.75 against 2.31 ms, 110 cells (10) 2.40 against
-// 2.46, 150 cells (14) 2.88 against 2.62.
+// 432 CRUs (5 warps per SM) 1.62 against 2.10 ms, 100 cells (9) 2.14 against
+// 2.21, 110 cells (10) 2.25 against 2.23, 150 cells (14) 2.61 against 2.35.
+// (Fewer and larger cells gain beyond that: twelve 80x16x8 cells, 16 warps per
+// SM, 1.95 against 2.16.)
 bool wide_cells(const rh_sim* s) {
   return s->sets[kNarrowSet].ntiles <= 10 * (int64_t)s->sm_count;
 }
 
-// Whether the narrow tiles are split over five warps (tile.cuh).  Only one
-// cell group in a second, mostly empty wave prefers one warp per tile (552
-// tiles of one FP64 cell: 6.90 against 7.37 ms per 100 steps); other groups'
-// tiles fill such a wave (540 tiles of two cells: split 5.61 against 6.69).
+// Whether the narrow tiles are split over five warps (tile.cuh): always but for
+// one cell group of more than a wave of them, whose last wave nothing else fills
+// (one FP64 cell, one warp per tile against split, 100 steps: 441 tiles 6.20 and
+// 4.94 ms, 539 tiles 6.46 and 6.75, 797 tiles 7.74 and 7.88, 1,539 tiles 12.73
+// and 13.48; 820 tiles of four cells 7.17 and 6.13).
 bool split_tiles(const rh_sim* s) {
   const int64_t tiles = s->sets[kNarrowSet].ntiles, wave = (int64_t)kSplitBlocks * s->sm_count;
-  return active_set(s) == kNarrowSet && (s->ngroups > 1 || tiles <= wave || tiles >= 2 * wave);
+  return active_set(s) == kNarrowSet && (s->ngroups > 1 || tiles <= wave);
 }
 
 // Staging of the FP32 lattice launches: the launch shape's, or while none was
 // asked for tensor copies from three waves of tiles on.  They take the own
 // planes' copies off the threads, which pays once CTAs follow one another
-// (per-thread against tensor copies, 100 steps: 512 cells 49.67 and 49.36 ms,
-// 256 cells 24.29 and 24.19, 60 cells 5.88 and 5.85), while in the first wave
-// their barrier initialisation and waits cost more (200 cells of 432 CRUs
-// 2.83 and 2.85 ms, 50 cells 1.73 and 1.75).  The same results.
+// (per-thread against tensor copies, means of eight runs of the same 100 steps,
+// which differ by 0.1 %: 512 cells 49.91 and 49.58 ms, 256 cells 24.86 and
+// 24.70, 128 cells 12.67 and 12.59, 60 cells 5.79 and 5.77), while in the first
+// waves their barrier initialisation and waits cost more (24 cells 2.36 and 2.40
+// ms, 200 cells of 432 CRUs 2.50 and 2.52).  The same results.
 int lattice_staging(const rh_sim* s) {
   if (split_tiles(s)) return 3;
   const int64_t wave = (int64_t)min_blocks_for<float, kDefaultTile>() * s->sm_count;
