@@ -205,7 +205,8 @@ cudaError_t launch_step(const StepArgs<R>& a, int ntiles, bool out, bool opt, in
   switch (tile) {
     case kNarrowTile:
       if (staging == 3) launch_bb<R, kNarrowTile, 3>(a, m, ntiles, out, opt, st);
-      else launch_bb<R, kNarrowTile, 0>(a, m, ntiles, out, opt, st);
+      else if constexpr (sizeof(R) == 8) launch_bb<R, kNarrowTile, 0>(a, m, ntiles, out, opt, st);
+      else return cudaErrorInvalidValue;  // FP32 narrow tiles are always split
       break;
     case 64: launch_b<R, 64>(a, m, ntiles, out, opt, staging, st); break;
     case 128: launch_b<R, 128>(a, m, ntiles, out, opt, staging, st); break;

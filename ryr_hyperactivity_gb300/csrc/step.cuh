@@ -13,7 +13,7 @@ constexpr int kNumTileSizes = 3;
 constexpr int kTileSizes[kNumTileSizes] = {64, 128, 256};
 constexpr int kDefaultTile = 128;
 
-// Narrow tiles, one or five warps per CTA, which the library uses by itself
+// Narrow tiles, five warps per CTA (or one, in FP64), which the library uses by itself
 // (they are no launch shape) where the default tiles would leave SMs idle or
 // unevenly loaded; the simulator keeps their tile table after the kTileSizes
 // ones.
@@ -35,7 +35,7 @@ constexpr int kDefaultGroups = 8;
 // so fewer, register-rich threads.
 template <class R, int B>
 __host__ __device__ constexpr int min_blocks_for() {
-  return sizeof(R) == 4 ? (B == 32 ? 20 : B == 64 ? 10 : (B == 128 ? 5 : 2))
+  return sizeof(R) == 4 ? (B == 64 ? 10 : (B == 128 ? 5 : 2))
                         : (B == 32 ? 12 : B == 64 ? 6 : (B == 128 ? 3 : 1));
 }
 
@@ -99,7 +99,7 @@ template <class R>
 cudaError_t window_grid(int tile, bool opt, bool fewer_ctas, int* ctas);
 
 // One time step with tiles of `tile` CRUs (one of kTileSizes, or kNarrowTile
-// with staging 0, or 3 for split tiles).  `opt` selects
+// with staging 3, split tiles, or in FP64 with 0).  `opt` selects
 // the kernel variant that handles the per-cell build options of the lattice
 // update (perm, iso, slowncxchange, NCX form); without them a cell runs the
 // plain variant.
