@@ -38,7 +38,8 @@ int rh_mlp_destroy(rh_mlp* m);
 int rh_mlp_param_count(const rh_mlp* m, int32_t* n);
 int rh_mlp_set_params(rh_mlp* m, const float* params);
 int rh_mlp_get_params(rh_mlp* m, float* params);
-/* y[n x 3] = network(x[n x 4]); any n (processed in batches of batch_max). */
+/* y[n x 3] = network(x[n x 4]); any n, in launches of 16,384 samples (or of
+ * batch_max, if that is more).  Arrays may lie at any address. */
 int rh_mlp_forward(rh_mlp* m, const float* x, int32_t n, float* y);
 /* Loss and parameter gradients for one batch (n <= batch_max); grads in the
  * parameter layout (may be NULL). */

@@ -491,8 +491,8 @@ __device__ __forceinline__ void image_from_params(const float* params, unsigned 
 //
 // What bounds it: a tile's arithmetic is a few microseconds of one SM's tensor
 // cores, so a pass is the latency of its layers, one after the other: an MMA
-// chain, a round trip to an mbarrier and an epilogue each (10 us forward, 13 us
-// a tile in training, plus 12 us for the weights and the gradients).  So the
+// chain, a round trip to an mbarrier and an epilogue each (11 us forward, 13 us
+// a tile in training, plus 14 us for the weights and the gradients).  So the
 // layers run in one CTA with the activations in shared memory.  One launch per
 // product, bias and activation, as before, cost 24 us of strided staging per
 // product (500 us for a dW over 4,096 samples in one CTA) and ten to 25
@@ -917,11 +917,12 @@ int reachable(rh_mlp* m, const float* p, size_t count, CopySlot slot, const floa
 }
 
 // One training pass: loss terms to h_out, each CTA's gradients to part.  A
-// batch of up to two tiles is one CTA's work, whose accumulators then hold
-// the whole batch's sums; a larger one is spread a tile to a CTA, and the
-// short accumulations and the ordered FP32 sum of the CTAs' gradients are more
-// exact than one accumulator over the batch (4,096 samples: median error
-// 8e-8 relative against 2e-6).
+// batch is spread a tile to a CTA; the short accumulations and the ordered FP32
+// sum of the CTAs' gradients are more exact than one accumulator over the batch
+// (4,096 samples: median error 8e-8 relative against 2e-6).  Up to two tiles
+// are one CTA's work: one accumulator, so that a step of the default batch of
+// 256 samples adds in the order in which it always has.  Two CTAs would save it
+// about 13 of 41 us and change that order.
 int train_pass(rh_mlp* m, const float* x, const float* target, int n, int* nparts) {
   const int tiles = (n + 127) / 128;
   *nparts = tiles <= 2 ? 1 : std::min(tiles, kMaxParts);

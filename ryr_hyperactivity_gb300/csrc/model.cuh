@@ -609,9 +609,9 @@ __device__ __forceinline__ void ryr_draws(rh_stream* rng, const StepCoef<R>& k, 
 //
 // A draw compares FP64 uniforms with FP64 rates; the outcome is an integer.
 // FP32 estimates of both sides decide it wherever they differ by more than
-// the estimates' error, and only a CRU with a closer comparison (about one
-// warp in a hundred has one) repeats its draws in FP64: the counts are those
-// of the FP64 comparison in every case.  That takes the eight exponentials,
+// the estimates' error, and only a CRU with a closer comparison (at the model's
+// step one in 10,000, so one to five warps in a thousand) repeats its draws in
+// FP64: the counts are those of the FP64 comparison in every case.  That takes the eight exponentials,
 // the rates' divisions and the uniforms' conversions off the FP64 pipe, which
 // bounds this kernel.
 

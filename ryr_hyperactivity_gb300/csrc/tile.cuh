@@ -181,10 +181,10 @@ __device__ __forceinline__ void cell_update(const StepArgs<R>& a, int cell, int 
 // only the old state, so nothing passes between the warps but the output
 // step's per-pair sums.  For lattices too small to fill the GPU, where a
 // step takes as long as one warp's instructions: in FP64 a warp issues one
-// FP64 instruction every 64 cycles, 1,170 of them for a whole tile, 420 at
-// most on any of the SM's four schedulers when split.  100 steps of one cell,
-// one warp per tile and split: 20x10x5 FP64 5.90 and 2.82 ms, 100x20x10 FP64
-// 6.40 and 5.30, 100x20x10 mixed 1.62 and 1.51.
+// FP64 instruction every 64 cycles, 1,050 of them for a whole tile, about 360
+// at most on any of the SM's four schedulers when split.  100 steps of one cell,
+// one warp per tile and split: 20x10x5 FP64 5.81 and 2.75 ms, 100x20x10 FP64
+// 6.17 and 4.95, 100x20x10 mixed 1.42 and 1.39.
 constexpr int kSplitWarps = 5;
 constexpr int kChannelWarp = 3;  // the pairs 0-3 are warps 0, 1, 2, 4
 // output-step sums of a pair and the statistics they belong to
