@@ -327,39 +327,34 @@ __device__ inline void wholecell_columns_warp(double* w, const double* o, const 
 // would be off by 14 times as much, over 5,100 by 25 times.  A warp's FP64
 // additions cost the same with one lane or 32, so a statistic per lane beats a
 // partial sum per lane with a reduction for each of the 33 statistics (441
-// rows: 480 additions against 630).  Eight groups of four partial sums, up
-// to 16 loads in flight, taken in the order in which the pairs of the tree
-// close, so that three pending sums are all that is kept.
+// rows: 472 additions against 630).  Four groups of eight partial sums, eight
+// loads in flight, taken in the order in which the pairs of the tree close, so
+// that two pending sums are all that is kept (eight groups of four with 16 loads
+// in flight, more code: a 20x10x5 FP64 cell's window 0.8 % longer).
 __device__ inline void output_sums_warp(const double* partials, int nrows, double* o, int lane) {
   static_assert(O_CIHIGH - P_STEP_END == NOUT - 1 && NOUT - 1 == 32, "one statistic per lane");
   const double* p = partials + P_STEP_END + lane;
-  double pending[3] = {0.0, 0.0, 0.0}, t = 0.0;
+  double pending[2] = {0.0, 0.0}, t = 0.0;
 #pragma unroll 1
-  for (int i = 0; i < 8; ++i) {
-    const int j = (int)(__brev((unsigned)i) >> 29);  // partial sums j, j + 8, j + 16, j + 24
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int i = 0; i < 4; ++i) {
+    const int j = (i & 1) * 2 + (i >> 1);  // partial sums j, j + 4, .. j + 28
+    double s[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll 1
-    for (int r = j; r < nrows; r += 128) {
-      double v[16];
+    for (int r = j; r < nrows; r += 32) {
+      double v[8];
 #pragma unroll
-      for (int q = 0; q < 16; ++q)
-        if (r + 8 * q < nrows) v[q] = __ldcg(p + (size_t)(r + 8 * q) * P_COUNT);
+      for (int q = 0; q < 8; ++q)
+        if (r + 4 * q < nrows) v[q] = __ldcg(p + (size_t)(r + 4 * q) * P_COUNT);
 #pragma unroll
-      for (int q = 0; q < 16; ++q)
-        if (r + 8 * q < nrows) s[q & 3] += v[q];
+      for (int q = 0; q < 8; ++q)
+        if (r + 4 * q < nrows) s[q] += v[q];
     }
-    t = (s[0] + s[2]) + (s[1] + s[3]);
-    bool open = true;
-#pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      if (open && (i >> b & 1)) {
-        t = pending[b] + t;
-      } else if (open) {
-        pending[b] = t;
-        open = false;
-      }
-    }
+    t = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+    if (i & 1) t = pending[0] + t;
+    else pending[0] = t;
+    if (i == 1) pending[1] = t;
   }
+  t = pending[1] + t;
   bool high = false;
   for (int r = lane; r < nrows; r += 32)
     high |= __ldcg(partials + (size_t)r * P_COUNT + O_CIHIGH) > 0.0;
