@@ -74,6 +74,14 @@ def init_params(seed: int = 0) -> np.ndarray:
     return np.concatenate(parts)
 
 
+def _rows(a: np.ndarray, n: int, width: int) -> np.ndarray:
+    """`a`, which must hold the n * width values that the GPU reads from its
+    memory: past its end there may be none."""
+    if a.size < n * width:
+        raise ValueError(f"{a.size} values where {n} samples take {n * width}")
+    return a
+
+
 class Surrogate:
     def __init__(self, batch_max: int = 4096, seed: int = 0, device: int = 0):
         self.L = _lib()
@@ -117,6 +125,7 @@ class Surrogate:
 
     def predict(self, x: np.ndarray) -> np.ndarray:
         x = np.ascontiguousarray(x, np.float32)
+        _rows(x, x.shape[0], N_IN)
         y = np.zeros((x.shape[0], N_OUT), np.float32)
         self._ck(self.L.rh_mlp_forward(self.h, _fptr(x), x.shape[0], _fptr(y)))
         return y
@@ -124,6 +133,8 @@ class Surrogate:
     def gradients(self, x: np.ndarray, t: np.ndarray):
         x = np.ascontiguousarray(x, np.float32)
         t = np.ascontiguousarray(t, np.float32)
+        _rows(x, x.shape[0], N_IN)
+        _rows(t, x.shape[0], N_OUT)
         g = np.zeros(self.nparams, np.float32)
         loss = C.c_float()
         self._ck(self.L.rh_mlp_gradients(self.h, _fptr(x), _fptr(t), x.shape[0], _fptr(g),
@@ -143,8 +154,8 @@ class Surrogate:
             tot, cnt = 0.0, 0
             for s in range(0, n - batch + 1, batch):
                 idx = order[s:s + batch]
-                xb = np.ascontiguousarray(x[idx])
-                tb = np.ascontiguousarray(t[idx])
+                xb = _rows(np.ascontiguousarray(x[idx]), batch, N_IN)
+                tb = _rows(np.ascontiguousarray(t[idx]), batch, N_OUT)
                 loss = C.c_float()
                 step_lr = lr * (0.5 * (1 + np.cos(np.pi * ep / epochs)))  # cosine schedule
                 self._ck(self.L.rh_mlp_train_step(self.h, _fptr(xb), _fptr(tb), batch,
