@@ -496,9 +496,9 @@ __device__ __forceinline__ void image_from_params(const float* params, unsigned 
 // layers run in one CTA with the activations in shared memory.  One launch per
 // product, bias and activation, as before, cost 24 us of strided staging per
 // product (500 us for a dW over 4,096 samples in one CTA) and ten to 25
-// launches.  Whole calls, before and now: 65,536 predictions 2.20 ms and 95 us,
-// an epoch of twelve 256-sample steps 5.50 and 0.86 ms, gradients of 4,096
-// samples 2.04 ms and 58 us, the no-allocation forward of 1,000 samples 61 and
+// launches.  Whole calls, before and now: 65,536 predictions 2.20 ms and 94 us,
+// an epoch of twelve 256-sample steps 5.50 and 0.83 ms, gradients of 4,096
+// samples 2.04 ms and 55 us, the no-allocation forward of 1,000 samples 61 and
 // 12 us.  256 threads (64 columns each) were slower: 44 us against 38 for two
 // training tiles.
 //

@@ -39,8 +39,7 @@ def normalise(points: np.ndarray) -> np.ndarray:
 
 def _lib():
     L = native.load()
-    vp = C.c_void_p
-    fp = C.POINTER(C.c_float)
+    vp = fp = C.c_void_p
     L.rh_mlp_create.argtypes = [C.c_int32, C.c_int32, C.POINTER(vp)]
     L.rh_mlp_destroy.argtypes = [vp]
     L.rh_mlp_param_count.argtypes = [vp, C.POINTER(C.c_int32)]
@@ -53,8 +52,8 @@ def _lib():
     return L
 
 
-def _fptr(a: np.ndarray):
-    return a.ctypes.data_as(C.POINTER(C.c_float))
+def _fptr(a: np.ndarray) -> int:
+    return a.ctypes.data  # the caller keeps `a` alive
 
 
 def init_params(seed: int = 0) -> np.ndarray:
